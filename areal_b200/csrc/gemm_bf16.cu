@@ -12,6 +12,7 @@
 #include "common/gemm_core.cuh"
 #include "common/host_utils.h"
 #include "common/io.cuh"
+#include "common/rms_row.cuh"
 
 namespace b200 {
 
@@ -390,74 +391,88 @@ __global__ void splitk_reduce_glu_kernel(const float* __restrict__ ws, __nv_bflo
 }
 
 // Split-K reduction fused with the residual add and RMSNorm that follow a projection in a decoder
-// block: one warp per row sums the S fp32 slices (+ bias), rounds to bf16 (the projection's output
-// precision), adds the bf16 residual stream, stores the new residual (bf16) and the normalised row.
-// Every rounding step of the unfused sequence (GEMM → bf16, residual add → bf16, norm) is kept, so
-// the results are bit-identical to it. N = 256 * NV at most (a lane owns NV groups of 8 columns).
-template <int NV>
-__global__ void splitk_reduce_rmsnorm_kernel(const float* __restrict__ ws, const __nv_bfloat16* __restrict__ bias,
-                                             const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
-                                             __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out,
-                                             int M, int N, int S, long long slice_stride, float eps) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
+// block: a group of threads per row (common/rms_row.cuh) sums the S fp32 slices (+ bias), rounds to bf16 (the
+// projection's output precision), adds the bf16 residual stream, stores the new residual (bf16) and the normalised row.
+// Every rounding step of the unfused sequence (GEMM → bf16, residual add → bf16, norm) is kept, as is the order of the
+// sum of squares, so the results are bit-identical to it. A decode step has few rows, so what counts is the chain of a
+// row: one warp walking over 2048 columns and up to 8 slices took 14 us for one row (4096 columns: 42 us); 256 threads with
+// the slices' loads side by side take 4.7 us (3.8 us).
+template <int VPT>
+__global__ void __launch_bounds__(512)
+splitk_reduce_rmsnorm_kernel(const float* __restrict__ ws, const __nv_bfloat16* __restrict__ bias,
+                             const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
+                             __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, int M, int N, int S,
+                             long long slice_stride, float eps) {
+  __shared__ float part[8][kRmsMaxWarps];
+  const int tid = threadIdx.x, group = blockDim.x;
+  const long long row = static_cast<long long>(blockIdx.x) * blockDim.y + threadIdx.y;
+  if (row >= M) return;  // the whole group
   const int nvec = N >> 3;
-  for (long long row = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); row < M;
-       row += static_cast<long long>(gridDim.x) * warps_per_block) {
-    float v[NV][8];
-    float ss = 0.f;
+  float v[VPT][8], ss = 0.f;
+  uint4 wraw[VPT];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < nvec) {
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int sl = 0; sl < S; ++sl) {
-          const float4* src = reinterpret_cast<const float4*>(ws + sl * slice_stride + row * N + c * 8);
-          const float4 a = src[0], b = src[1];
-          acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-          acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-        }
-        if (bias) {
+  for (int i = 0; i < VPT; ++i) {
+    const int c = tid + group * i;
+    if (c < nvec) {
+      wraw[i] = reinterpret_cast<const uint4*>(w)[c];
+      uint4 rraw = res ? reinterpret_cast<const uint4*>(res + row * N)[c] : make_uint4(0, 0, 0, 0);
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const float* base = ws + row * N + c * 8;
+      for (int s0 = 0; s0 < S; s0 += 4) {
+        float4 a[4], b[4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += __bfloat162float(bias[c * 8 + j]);
+        for (int u = 0; u < 4; ++u) {
+          if (s0 + u < S) {
+            const float4* src = reinterpret_cast<const float4*>(base + (s0 + u) * slice_stride);
+            a[u] = src[0];
+            b[u] = src[1];
+          } else {
+            a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
-        uint4 rraw = res ? reinterpret_cast<const uint4*>(res + row * N)[c] : make_uint4(0, 0, 0, 0);
-        const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rraw);
-        uint4 hraw;
-        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&hraw);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // projection output in bf16, then the residual add in fp32, then the bf16 residual stream
-          const float2 a2 = __bfloat1622float2(__floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]));
-          const float2 r2 = __bfloat1622float2(rp[j]);
-          hp[j] = res ? __floats2bfloat162_rn(a2.x + r2.x, a2.y + r2.y) : __floats2bfloat162_rn(a2.x, a2.y);
-          const float2 h2 = __bfloat1622float2(hp[j]);
-          v[i][2 * j] = h2.x;
-          v[i][2 * j + 1] = h2.y;
-          ss += h2.x * h2.x;  // same accumulation order as the stand-alone RMSNorm kernel
-          ss += h2.y * h2.y;
+        for (int u = 0; u < 4; ++u) {
+          acc[0] += a[u].x; acc[1] += a[u].y; acc[2] += a[u].z; acc[3] += a[u].w;
+          acc[4] += b[u].x; acc[5] += b[u].y; acc[6] += b[u].z; acc[7] += b[u].w;
         }
-        reinterpret_cast<uint4*>(res_out + row * N)[c] = hraw;
       }
+      if (bias) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += __bfloat162float(bias[c * 8 + j]);
+      }
+      const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rraw);
+      uint4 hraw;
+      __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&hraw);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // projection output in bf16, then the residual add in fp32, then the bf16 residual stream
+        const float2 a2 = __bfloat1622float2(__floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]));
+        const float2 r2 = __bfloat1622float2(rp[j]);
+        hp[j] = res ? __floats2bfloat162_rn(a2.x + r2.x, a2.y + r2.y) : __floats2bfloat162_rn(a2.x, a2.y);
+        const float2 h2 = __bfloat1622float2(hp[j]);
+        v[i][2 * j] = h2.x;
+        v[i][2 * j + 1] = h2.y;
+        ss += h2.x * h2.x;  // same accumulation order as the stand-alone RMSNorm kernel
+        ss += h2.y * h2.y;
+      }
+      reinterpret_cast<uint4*>(res_out + row * N)[c] = hraw;
     }
+  }
+  ss = rms_group_sum(ss, part[threadIdx.y], tid, group, threadIdx.y);
+  const float rs = rsqrtf(ss / N + eps);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rs = rsqrtf(ss / N + eps);
+  for (int i = 0; i < VPT; ++i) {
+    const int c = tid + group * i;
+    if (c < nvec) {
+      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wraw[i]);
+      uint4 oraw;
+      __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < nvec) {
-        const uint4 wraw = reinterpret_cast<const uint4*>(w)[c];
-        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wraw);
-        uint4 oraw;
-        __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&oraw);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 w2 = __bfloat1622float2(wp[j]);
-          op[j] = __floats2bfloat162_rn(v[i][2 * j] * rs * w2.x, v[i][2 * j + 1] * rs * w2.y);
-        }
-        reinterpret_cast<uint4*>(y + row * N)[c] = oraw;
+      for (int j = 0; j < 4; ++j) {
+        const float2 w2 = __bfloat1622float2(wp[j]);
+        op[j] = __floats2bfloat162_rn(v[i][2 * j] * rs * w2.x, v[i][2 * j + 1] * rs * w2.y);
       }
+      reinterpret_cast<uint4*>(y + row * N)[c] = oraw;
     }
   }
 }
@@ -767,19 +782,14 @@ int b200_gemm_bf16_splitk_rmsnorm(const void* A, const void* B, const void* bias
   long long stride = 0;
   const int rc = launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, &S, &stride, stream);
   if (rc) return rc;
-  const int nv = (N / 8 + 31) / 32;
-  const int wpb = 8;
-  const unsigned grid = static_cast<unsigned>((M + wpb - 1) / wpb);
-#define B200_LAUNCH_RN(NV_)                                                                                  \
-  splitk_reduce_rmsnorm_kernel<NV_><<<grid, wpb * 32, 0, stream>>>(                                          \
+  const RmsShape shape = rms_shape(N);
+  const int rows = 256 / shape.group > 1 ? 256 / shape.group : 1;
+#define B200_LAUNCH_RN(VPT_)                                                                                 \
+  splitk_reduce_rmsnorm_kernel<VPT_><<<(M + rows - 1) / rows, dim3(shape.group, rows), 0, stream>>>(         \
       workspace, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)norm_w,   \
       (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, M, N, S, stride, eps)
-  if (nv <= 1) B200_LAUNCH_RN(1);
-  else if (nv <= 2) B200_LAUNCH_RN(2);
-  else if (nv <= 4) B200_LAUNCH_RN(4);
-  else if (nv <= 8) B200_LAUNCH_RN(8);
-  else if (nv <= 16) B200_LAUNCH_RN(16);
-  else B200_LAUNCH_RN(32);
+  if (shape.vpt == 1) B200_LAUNCH_RN(1);
+  else B200_LAUNCH_RN(2);
 #undef B200_LAUNCH_RN
   B200_CHECK(cudaGetLastError());
   return 0;

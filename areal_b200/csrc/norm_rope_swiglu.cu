@@ -8,6 +8,7 @@
 // 103-293; qwen2/model/rope.py).
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "norm_static_scratch.h"
 #include <cuda_bf16.h>
@@ -15,6 +16,7 @@
 #include <stdint.h>
 
 #include "common/host_utils.h"
+#include "common/rms_row.cuh"
 
 namespace b200 {
 
@@ -43,383 +45,535 @@ __device__ __forceinline__ BF8 float_to_bf8(const float* f) {
 }
 
 // ------------------------------------------------------------------ RMSNorm --
-// One warp per row; a lane holds NV 16-byte vectors (8 bf16 each), so the row
-// (H = 256 * NV elements at most) is read once.
-template <int NV>
-__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                   const __nv_bfloat16* __restrict__ res,
-                                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                   __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd,
-                                   int T, int H, float eps) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
+// A group of threads per row (common/rms_row.cuh), blockDim = (group, groups of the block). Bound by memory: x, the residual
+// and both results cross HBM once. With a warp a row and 64 columns a lane, 16384 x 2048 with residual took 64 us (4.2 TB/s);
+// spread over 256 threads it takes as long with one row a group, which leaves memory idle between blocks, and 53 us (5.1
+// TB/s) with two rows a group, loaded together (four: 53 us). 32768 x 4096: 359 us before, 196 us now.
+template <int VPT, int ROWS>
+__global__ void __launch_bounds__(512)
+rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                   __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int T, int H, float eps) {
+  __shared__ float part[8][ROWS][kRmsMaxWarps];
+  const int tid = threadIdx.x, group = blockDim.x;
+  const long long row0 = (static_cast<long long>(blockIdx.x) * blockDim.y + threadIdx.y) * ROWS;
+  if (row0 >= T) return;  // the whole group
   const int nvec = H >> 3;
-  for (long long row = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5);
-       row < T; row += static_cast<long long>(gridDim.x) * warps_per_block) {
-    const BF8* xr = reinterpret_cast<const BF8*>(x + row * H);
-    const BF8* rr = res ? reinterpret_cast<const BF8*>(res + row * H) : nullptr;
-    float v[NV][8];
-    float ss = 0.f;
+  BF8 h[ROWS][VPT], r[ROWS][VPT];
+  float ss[ROWS];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < nvec) {
-        bf8_to_float(xr[c], v[i]);
-        if (rr) {
-          float r[8];
-          bf8_to_float(rr[c], r);
+  for (int k = 0; k < ROWS; ++k)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[i][j] += r[j];
-          // the residual stream is kept in bf16: normalise what is stored
-          BF8 h = float_to_bf8(v[i]);
-          reinterpret_cast<BF8*>(res_out + row * H)[c] = h;
-          bf8_to_float(h, v[i]);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
+    for (int i = 0; i < VPT; ++i) {
+      const int c = tid + group * i;
+      if (c < nvec && row0 + k < T) {
+        h[k][i] = reinterpret_cast<const BF8*>(x + (row0 + k) * H)[c];
+        if (res) r[k][i] = reinterpret_cast<const BF8*>(res + (row0 + k) * H)[c];
       }
     }
-    ss = warp_sum(ss);
-    const float rs = rsqrtf(ss / H + eps);
-    if (lane == 0 && rstd) rstd[row] = rs;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < nvec) {
-        float wv[8];
-        bf8_to_float(reinterpret_cast<const BF8*>(w)[c], wv);
-        float o[8];
+  for (int k = 0; k < ROWS; ++k) {
+    ss[k] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = v[i][j] * rs * wv[j];
-        reinterpret_cast<BF8*>(y + row * H)[c] = float_to_bf8(o);
+    for (int i = 0; i < VPT; ++i) {
+      const int c = tid + group * i;
+      if (c < nvec && row0 + k < T) {
+        float v[8];
+        bf8_to_float(h[k][i], v);
+        if (res) {
+          float f[8];
+          bf8_to_float(r[k][i], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += f[j];
+          // the residual stream is kept in bf16: normalise what is stored
+          h[k][i] = float_to_bf8(v);
+          reinterpret_cast<BF8*>(res_out + (row0 + k) * H)[c] = h[k][i];
+          bf8_to_float(h[k][i], v);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss[k] += v[j] * v[j];
       }
+    }
+  }
+  rms_group_sums<ROWS>(ss, &part[threadIdx.y][0][0], tid, group, threadIdx.y);
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = tid + group * i;
+    if (c < nvec) {
+      float f[8];
+      bf8_to_float(reinterpret_cast<const BF8*>(w)[c], f);
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k)
+        if (row0 + k < T) {
+          const float rs = rsqrtf(ss[k] / H + eps);
+          if (tid == 0 && i == 0 && rstd) rstd[row0 + k] = rs;
+          float v[8], o[8];
+          bf8_to_float(h[k][i], v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = v[j] * rs * f[j];
+          reinterpret_cast<BF8*>(y + (row0 + k) * H)[c] = float_to_bf8(o);
+        }
     }
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres); dw partial per block.
-template <int NV>
-__global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                   const __nv_bfloat16* __restrict__ x,
-                                   const __nv_bfloat16* __restrict__ w,
-                                   const float* __restrict__ rstd,
-                                   const __nv_bfloat16* __restrict__ dres,
-                                   __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
-                                   int T, int H) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres); one partial row of dw per block. A thread keeps its columns over all
+// rows of its group, so dw accumulates in registers; the next row is loaded before the current one is reduced, so that
+// the barrier of the sum does not leave memory idle. 16384 x 2048: 164 us with a warp a row (8 vectors a lane and no
+// load ahead), 80 us so; 32768 x 4096: 1050 us and 297 us.
+template <int VPT>
+__global__ void __launch_bounds__(512)
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
+                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                   float* __restrict__ dw_partial, int T, int H) {
+  __shared__ float part[2][8][kRmsMaxWarps];
+  extern __shared__ float sm[];  // [rows of the block - 1][H], only with more than one
+  const int tid = threadIdx.x, group = blockDim.x, slot = threadIdx.y;
   const int nvec = H >> 3;
-  float dwacc[NV][8];
+  const float inv_h = 1.f / H;
+  float wv[VPT][8], dwacc[VPT][8];
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
+  for (int i = 0; i < VPT; ++i) {
+    const int c = tid + group * i;
+    if (c < nvec) bf8_to_float(reinterpret_cast<const BF8*>(w)[c], wv[i]);
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-  float wv[NV][8];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = lane + 32 * i;
-    if (c < nvec) bf8_to_float(reinterpret_cast<const BF8*>(w)[c], wv[i]);
   }
-  for (long long row = static_cast<long long>(blockIdx.x) * warps_per_block + warp; row < T;
-       row += static_cast<long long>(gridDim.x) * warps_per_block) {
-    const float rs = rstd[row];
-    float g[NV][8], xh[NV][8];
-    float dot = 0.f;
+  struct Row {
+    BF8 g[VPT], x[VPT], r[VPT];
+    float rs;
+  };
+  auto load = [&](long long row, Row& o) {
+    o.rs = rstd[row];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
+    for (int i = 0; i < VPT; ++i) {
+      const int c = tid + group * i;
       if (c < nvec) {
-        bf8_to_float(reinterpret_cast<const BF8*>(dy + row * H)[c], g[i]);
-        bf8_to_float(reinterpret_cast<const BF8*>(x + row * H)[c], xh[i]);
+        o.g[i] = reinterpret_cast<const BF8*>(dy + row * H)[c];
+        o.x[i] = reinterpret_cast<const BF8*>(x + row * H)[c];
+        if (dres) o.r[i] = reinterpret_cast<const BF8*>(dres + row * H)[c];
+      }
+    }
+  };
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.y;
+  long long row = static_cast<long long>(blockIdx.x) * blockDim.y + slot;
+  Row cur, nxt;
+  if (row < T) load(row, cur);
+  for (int it = 0; row < T; row += step, ++it) {
+    if (row + step < T) load(row + step, nxt);
+    float g[VPT][8], xh[VPT][8], dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      if (tid + group * i < nvec) {
+        bf8_to_float(cur.g[i], g[i]);
+        bf8_to_float(cur.x[i], xh[i]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] *= rs;
+          xh[i][j] *= cur.rs;
           dwacc[i][j] += g[i][j] * xh[i][j];
           g[i][j] *= wv[i][j];
           dot += g[i][j] * xh[i][j];
         }
       }
     }
-    dot = warp_sum(dot) / H;
+    dot = rms_group_sum(dot, part[it & 1][slot], tid, group, slot) * inv_h;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
+    for (int i = 0; i < VPT; ++i) {
+      const int c = tid + group * i;
       if (c < nvec) {
         float o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (g[i][j] - xh[i][j] * dot);
+        for (int j = 0; j < 8; ++j) o[j] = cur.rs * (g[i][j] - xh[i][j] * dot);
         if (dres) {
           float r[8];
-          bf8_to_float(reinterpret_cast<const BF8*>(dres + row * H)[c], r);
+          bf8_to_float(cur.r[i], r);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += r[j];
         }
         reinterpret_cast<BF8*>(dx + row * H)[c] = float_to_bf8(o);
       }
     }
+    cur = nxt;
   }
-  // reduce the per-warp dw accumulators across the block through shared memory
-  extern __shared__ float sm[];  // [warps][H]
+  // the block's row groups meet in shared memory
+  if (blockDim.y > 1) {
+    if (slot) {
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = lane + 32 * i;
-    if (c < nvec)
+      for (int i = 0; i < VPT; ++i) {
+        const int c = tid + group * i;
+        if (c < nvec)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) sm[warp * H + c * 8 + j] = dwacc[i][j];
+          for (int j = 0; j < 8; ++j) sm[(slot - 1) * H + c * 8 + j] = dwacc[i][j];
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int c = threadIdx.x; c < H; c += blockDim.x) {
-    float s = 0.f;
-    for (int wi = 0; wi < warps_per_block; ++wi) s += sm[wi * H + c];
-    dw_partial[static_cast<long long>(blockIdx.x) * H + c] = s;
+  if (slot) return;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = tid + group * i;
+    if (c < nvec) {
+      for (int s = 1; s < blockDim.y; ++s)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dwacc[i][j] += sm[(s - 1) * H + c * 8 + j];
+      float4* out = reinterpret_cast<float4*>(dw_partial + static_cast<long long>(blockIdx.x) * H + c * 8);
+      out[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+      out[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
+    }
   }
 }
 
-__global__ void colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                                       int nblocks, int H, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
+// Column sums of the partial rows: 32 columns a block, its 16 warps take every 16th row. (With one thread a column
+// walking all rows this took 12 us, with these 5 us.)
+__global__ void __launch_bounds__(512)
+colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int nblocks, int H,
+                       int accumulate) {
+  __shared__ float sm[16][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int b = 0; b < nblocks; ++b) s += partial[static_cast<long long>(b) * H + c];
+  if (c < H)
+#pragma unroll 4
+    for (int b = warp; b < nblocks; b += 16) s += partial[static_cast<long long>(b) * H + c];
+  sm[warp][lane] = s;
+  __syncthreads();
+  if (warp || c >= H) return;
+#pragma unroll
+  for (int i = 1; i < 16; ++i) s += sm[i][lane];
   out[c] = accumulate ? out[c] + s : s;
 }
 
 // ------------------------------------------------------- q/k norm + RoPE ----
-// qkv: [T, (Hq + 2*Hkv) * D] bf16 (q heads, then k heads, then v heads).
-// One warp per (token, head) over the q and k heads; D == 128 (lane owns the
-// pairs j = 2*lane, 2*lane+1 and their partners j + 64).
-__global__ void qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv,
-                                       const __nv_bfloat16* __restrict__ qw,
-                                       const __nv_bfloat16* __restrict__ kw,
-                                       const float* __restrict__ cos_t,
-                                       const float* __restrict__ sin_t,
-                                       const int* __restrict__ pos, __nv_bfloat16* __restrict__ q_out,
-                                       __nv_bfloat16* __restrict__ k_out, float* __restrict__ rstd_out,
-                                       int T, int Hq, int Hkv, float eps, int has_norm) {
-  constexpr int D = 128;
-  const int lane = threadIdx.x & 31;
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int heads = Hq + Hkv;
-  if (gw >= static_cast<long long>(T) * heads) return;
-  const int t = static_cast<int>(gw / heads);
-  const int h = static_cast<int>(gw % heads);
-  const long long row_stride = static_cast<long long>(Hq + 2 * Hkv) * D;
-  const __nv_bfloat16* src = qkv + t * row_stride + static_cast<long long>(h) * D;
-  const bool is_q = h < Hq;
-  const __nv_bfloat16* w = is_q ? qw : kw;
-  __nv_bfloat16* dst = is_q ? q_out + (static_cast<long long>(t) * Hq + h) * D
-                            : k_out + (static_cast<long long>(t) * Hkv + (h - Hq)) * D;
-  float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src)[lane]);
-  float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src + 64)[lane]);
-  if (has_norm) {
-    float ss = warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
-    const float rs = rsqrtf(ss / D + eps);
-    if (lane == 0) rstd_out[gw] = rs;
-    float2 wa = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w)[lane]);
-    float2 wb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w + 64)[lane]);
-    // match the reference's rounding: the normalised value is cast to bf16 before RoPE
-    a.x = __bfloat162float(__float2bfloat16(a.x * rs * wa.x));
-    a.y = __bfloat162float(__float2bfloat16(a.y * rs * wa.y));
-    b.x = __bfloat162float(__float2bfloat16(b.x * rs * wb.x));
-    b.y = __bfloat162float(__float2bfloat16(b.y * rs * wb.y));
+// qkv: [T, (Hq + 2*Hkv) * D] bf16 (q heads, then k heads, then v heads), D == 128. Eight lanes share a head: a lane owns
+// columns 8l..8l+7 and their partners 64 + 8l.. (16-byte vectors), so a warp works on four heads of a token at a time,
+// the sum of squares takes three shuffles, and the token's angles are read once for all of them. With a warp a head and four columns
+// a lane the kernels were bound by issue slots: 16384 tokens of 16 + 8 heads took 91 us forward and 172 us backward, now
+// 51 and 143 us (the latter with the copy of dv, which was a launch of its own).
+constexpr int kRopeD = 128;
+constexpr int kRopeHeads = 4;  // heads of a warp at a time
+
+struct RopeVec {  // a lane's columns of one head
+  float a[8], b[8];
+  __device__ __forceinline__ void read(const __nv_bfloat16* p, int l) {
+    bf8_to_float(reinterpret_cast<const BF8*>(p)[l], a);
+    bf8_to_float(reinterpret_cast<const BF8*>(p + 64)[l], b);
   }
-  const int p = pos[t];
-  const float2 c = reinterpret_cast<const float2*>(cos_t + static_cast<long long>(p) * 64)[lane];
-  const float2 s = reinterpret_cast<const float2*>(sin_t + static_cast<long long>(p) * 64)[lane];
-  float2 oa, ob;
-  oa.x = a.x * c.x - b.x * s.x;
-  oa.y = a.y * c.y - b.y * s.y;
-  ob.x = b.x * c.x + a.x * s.x;
-  ob.y = b.y * c.y + a.y * s.y;
-  reinterpret_cast<__nv_bfloat162*>(dst)[lane] = __floats2bfloat162_rn(oa.x, oa.y);
-  reinterpret_cast<__nv_bfloat162*>(dst + 64)[lane] = __floats2bfloat162_rn(ob.x, ob.y);
+  __device__ __forceinline__ void write(__nv_bfloat16* p, int l) const {
+    reinterpret_cast<BF8*>(p)[l] = float_to_bf8(a);
+    reinterpret_cast<BF8*>(p + 64)[l] = float_to_bf8(b);
+  }
+};
+
+struct RopeAngles {  // a lane's angles of one position
+  float c[8], s[8];
+  __device__ __forceinline__ void read(const float* __restrict__ cos_t, const float* __restrict__ sin_t, int p, int l) {
+    const float4* pc = reinterpret_cast<const float4*>(cos_t + static_cast<long long>(p) * 64) + 2 * l;
+    const float4* ps = reinterpret_cast<const float4*>(sin_t + static_cast<long long>(p) * 64) + 2 * l;
+    *reinterpret_cast<float4*>(c) = pc[0];
+    *reinterpret_cast<float4*>(c + 4) = pc[1];
+    *reinterpret_cast<float4*>(s) = ps[0];
+    *reinterpret_cast<float4*>(s + 4) = ps[1];
+  }
+};
+
+__device__ __forceinline__ float rope_sum8(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Norm (when w is given) and rotation of one head in place; returns the head's 1 / rms. Every lane of the warp calls.
+__device__ __forceinline__ float rope_head(RopeVec& v, const RopeAngles& r, const __nv_bfloat16* w, int l, float eps) {
+  float rs = 1.f;
+  if (w) {
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v.a[j] * v.a[j] + v.b[j] * v.b[j];
+    rs = rsqrtf(rope_sum8(ss) / kRopeD + eps);
+    RopeVec ww;
+    ww.read(w, l);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      // match the reference's rounding: the normalised value is cast to bf16 before RoPE
+      v.a[j] = __bfloat162float(__float2bfloat16(v.a[j] * rs * ww.a[j]));
+      v.b[j] = __bfloat162float(__float2bfloat16(v.b[j] * rs * ww.b[j]));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float a = v.a[j], b = v.b[j];
+    v.a[j] = a * r.c[j] - b * r.s[j];
+    v.b[j] = b * r.c[j] + a * r.s[j];
+  }
+  return rs;
+}
+
+__global__ void __launch_bounds__(256)
+qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qw,
+                       const __nv_bfloat16* __restrict__ kw, const float* __restrict__ cos_t,
+                       const float* __restrict__ sin_t, const int* __restrict__ pos,
+                       __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_out,
+                       float* __restrict__ rstd_out, int T, int Hq, int Hkv, float eps, int has_norm) {
+  constexpr int D = kRopeD, J = 2;  // a warp takes J rounds of kRopeHeads heads of one token
+  const int lane = threadIdx.x & 31, l = lane & 7;
+  const int heads = Hq + Hkv;
+  const int groups = (heads + J * kRopeHeads - 1) / (J * kRopeHeads);
+  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (gw >= static_cast<long long>(T) * groups) return;
+  const int t = static_cast<int>(gw / groups);
+  const int h0 = static_cast<int>(gw % groups) * J * kRopeHeads + (lane >> 3);
+  const __nv_bfloat16* src = qkv + static_cast<long long>(t) * (Hq + 2 * Hkv) * D;
+  RopeAngles ang;
+  ang.read(cos_t, sin_t, pos[t], l);
+  RopeVec v[J];
+#pragma unroll
+  for (int j = 0; j < J; ++j)  // lanes past the last head repeat it and write nothing
+    v[j].read(src + static_cast<long long>(min(h0 + j * kRopeHeads, heads - 1)) * D, l);
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const int h = h0 + j * kRopeHeads;
+    const bool is_q = h < Hq;
+    const float rs = rope_head(v[j], ang, has_norm ? (is_q ? qw : kw) : nullptr, l, eps);
+    if (h >= heads) continue;
+    if (has_norm && l == 0) rstd_out[static_cast<long long>(t) * heads + h] = rs;
+    v[j].write(is_q ? q_out + (static_cast<long long>(t) * Hq + h) * D
+                    : k_out + (static_cast<long long>(t) * Hkv + (h - Hq)) * D, l);
+  }
 }
 
 // Decode / prefill form of the kernel above: q is written out as before, k goes straight into the
 // paged K cache and v is copied into the paged V cache (`[page, kv head, slot in page, D]`), so the
-// separate cache-write launch disappears. One warp per (token, head) over q, k AND v heads.
+// separate cache-write launch disappears. A warp takes four of a token's q, k AND v heads.
 // slot_mapping[t] = page * block_size + offset, negative to skip the token's cache write.
-__global__ void qknorm_rope_kvwrite_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qw,
-                                           const __nv_bfloat16* __restrict__ kw, const float* __restrict__ cos_t,
-                                           const float* __restrict__ sin_t, const int* __restrict__ pos,
-                                           __nv_bfloat16* __restrict__ q_out,
-                                           const long long* __restrict__ slot_mapping,
-                                           __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
-                                           int T, int Hq, int Hkv, int block_size, float eps, int has_norm) {
-  constexpr int D = 128;
-  const int lane = threadIdx.x & 31;
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+__global__ void __launch_bounds__(128)
+qknorm_rope_kvwrite_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qw,
+                           const __nv_bfloat16* __restrict__ kw, const float* __restrict__ cos_t,
+                           const float* __restrict__ sin_t, const int* __restrict__ pos,
+                           __nv_bfloat16* __restrict__ q_out, const long long* __restrict__ slot_mapping,
+                           __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int T,
+                           int Hq, int Hkv, int block_size, float eps, int has_norm) {
+  constexpr int D = kRopeD;
+  const int lane = threadIdx.x & 31, l = lane & 7;
   const int heads = Hq + 2 * Hkv;
-  if (gw >= static_cast<long long>(T) * heads) return;
-  const int t = static_cast<int>(gw / heads);
-  const int h = static_cast<int>(gw % heads);
-  const __nv_bfloat16* src = qkv + (static_cast<long long>(t) * heads + h) * D;
-  const bool is_q = h < Hq;
-  const bool is_v = h >= Hq + Hkv;
-  __nv_bfloat16* dst;
-  if (is_q) {
-    dst = q_out + (static_cast<long long>(t) * Hq + h) * D;
-  } else {
-    const long long slot = slot_mapping[t];
-    if (slot < 0) return;
-    const long long blk = slot / block_size, off = slot % block_size;
-    const int hk = is_v ? h - Hq - Hkv : h - Hq;
-    dst = (is_v ? v_cache : k_cache) + ((blk * Hkv + hk) * block_size + off) * D;
-  }
-  if (is_v) {
-    reinterpret_cast<uint2*>(dst)[lane] = reinterpret_cast<const uint2*>(src)[lane];
+  const int groups = (heads + kRopeHeads - 1) / kRopeHeads;
+  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (gw >= static_cast<long long>(T) * groups) return;
+  const int t = static_cast<int>(gw / groups);
+  const int h = static_cast<int>(gw % groups) * kRopeHeads + (lane >> 3);
+  const int hs = min(h, heads - 1);
+  const long long slot = slot_mapping[t];
+  const __nv_bfloat16* src = qkv + (static_cast<long long>(t) * heads + hs) * D;
+  const BF8 raw_a = reinterpret_cast<const BF8*>(src)[l], raw_b = reinterpret_cast<const BF8*>(src + 64)[l];
+  RopeAngles ang;
+  ang.read(cos_t, sin_t, pos[t], l);
+  RopeVec v;
+  bf8_to_float(raw_a, v.a);
+  bf8_to_float(raw_b, v.b);
+  rope_head(v, ang, has_norm ? (hs < Hq ? qw : kw) : nullptr, l, eps);  // the result of a v head is not used
+  if (h >= heads) return;
+  if (h < Hq) {
+    v.write(q_out + (static_cast<long long>(t) * Hq + h) * D, l);
     return;
   }
-  const __nv_bfloat16* w = is_q ? qw : kw;
-  float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src)[lane]);
-  float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src + 64)[lane]);
-  if (has_norm) {
-    float ss = warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
-    const float rs = rsqrtf(ss / D + eps);
-    float2 wa = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w)[lane]);
-    float2 wb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w + 64)[lane]);
-    a.x = __bfloat162float(__float2bfloat16(a.x * rs * wa.x));
-    a.y = __bfloat162float(__float2bfloat16(a.y * rs * wa.y));
-    b.x = __bfloat162float(__float2bfloat16(b.x * rs * wb.x));
-    b.y = __bfloat162float(__float2bfloat16(b.y * rs * wb.y));
+  if (slot < 0) return;
+  const bool is_v = h >= Hq + Hkv;
+  const int hk = is_v ? h - Hq - Hkv : h - Hq;
+  __nv_bfloat16* dst = (is_v ? v_cache : k_cache) +
+                       (((slot / block_size) * Hkv + hk) * block_size + slot % block_size) * D;
+  if (is_v) {
+    reinterpret_cast<BF8*>(dst)[l] = raw_a;
+    reinterpret_cast<BF8*>(dst + 64)[l] = raw_b;
+  } else {
+    v.write(dst, l);
   }
-  const int p = pos[t];
-  const float2 c = reinterpret_cast<const float2*>(cos_t + static_cast<long long>(p) * 64)[lane];
-  const float2 s = reinterpret_cast<const float2*>(sin_t + static_cast<long long>(p) * 64)[lane];
-  float2 oa, ob;
-  oa.x = a.x * c.x - b.x * s.x;
-  oa.y = a.y * c.y - b.y * s.y;
-  ob.x = b.x * c.x + a.x * s.x;
-  ob.y = b.y * c.y + a.y * s.y;
-  reinterpret_cast<__nv_bfloat162*>(dst)[lane] = __floats2bfloat162_rn(oa.x, oa.y);
-  reinterpret_cast<__nv_bfloat162*>(dst + 64)[lane] = __floats2bfloat162_rn(ob.x, ob.y);
 }
 
-// Backward: un-rotate dq/dk, then per-head RMSNorm backward; writes into the
-// q and k slots of dqkv and accumulates dqw / dkw [D] with atomics (fp32).
-__global__ void qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq,
-                                       const __nv_bfloat16* __restrict__ dk,
-                                       const __nv_bfloat16* __restrict__ qkv,
-                                       const __nv_bfloat16* __restrict__ qw,
-                                       const __nv_bfloat16* __restrict__ kw,
-                                       const float* __restrict__ cos_t,
-                                       const float* __restrict__ sin_t,
-                                       const int* __restrict__ pos, const float* __restrict__ rstd,
-                                       __nv_bfloat16* __restrict__ dqkv, float* __restrict__ dqw,
-                                       float* __restrict__ dkw, int T, int Hq, int Hkv, int has_norm) {
-  constexpr int D = 128;
+// Backward: un-rotate dq/dk, then per-head RMSNorm backward; writes the q, k and (copied from dv) v slots of dqkv. A warp
+// keeps its heads and walks over tokens, so dqw / dkw [D] accumulate in registers and reach memory with one atomic
+// per column and block.
+__global__ void __launch_bounds__(256)
+qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk,
+                       const __nv_bfloat16* __restrict__ dv, const __nv_bfloat16* __restrict__ qkv,
+                       const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
+                       const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                       const int* __restrict__ pos, const float* __restrict__ rstd,
+                       __nv_bfloat16* __restrict__ dqkv, float* __restrict__ dqw, float* __restrict__ dkw,
+                       int T, int Hq, int Hkv, int has_norm) {
+  constexpr int D = kRopeD;
   __shared__ float s_dw[2][D];
   for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&s_dw[0][0])[i] = 0.f;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int heads = Hq + Hkv;
-  if (gw < static_cast<long long>(T) * heads) {
-    const int t = static_cast<int>(gw / heads);
-    const int h = static_cast<int>(gw % heads);
-    const bool is_q = h < Hq;
-    const long long row_stride = static_cast<long long>(Hq + 2 * Hkv) * D;
-    const __nv_bfloat16* g = is_q ? dq + (static_cast<long long>(t) * Hq + h) * D
-                                  : dk + (static_cast<long long>(t) * Hkv + (h - Hq)) * D;
-    float2 ga = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(g)[lane]);
-    float2 gb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(g + 64)[lane]);
-    const int p = pos[t];
-    const float2 c = reinterpret_cast<const float2*>(cos_t + static_cast<long long>(p) * 64)[lane];
-    const float2 s = reinterpret_cast<const float2*>(sin_t + static_cast<long long>(p) * 64)[lane];
-    // transpose of the rotation
-    float2 da, db;
-    da.x = ga.x * c.x + gb.x * s.x;
-    da.y = ga.y * c.y + gb.y * s.y;
-    db.x = gb.x * c.x - ga.x * s.x;
-    db.y = gb.y * c.y - ga.y * s.y;
-    __nv_bfloat16* out = dqkv + t * row_stride + static_cast<long long>(h) * D;
-    if (has_norm) {
-      const __nv_bfloat16* src = qkv + t * row_stride + static_cast<long long>(h) * D;
-      const __nv_bfloat16* w = is_q ? qw : kw;
-      float2 xa = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src)[lane]);
-      float2 xb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(src + 64)[lane]);
-      float2 wa = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w)[lane]);
-      float2 wb = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(w + 64)[lane]);
-      const float rs = rstd[gw];
-      xa.x *= rs; xa.y *= rs; xb.x *= rs; xb.y *= rs;
-      float* sw = s_dw[is_q ? 0 : 1];
-      atomicAdd(&sw[2 * lane], da.x * xa.x);
-      atomicAdd(&sw[2 * lane + 1], da.y * xa.y);
-      atomicAdd(&sw[64 + 2 * lane], db.x * xb.x);
-      atomicAdd(&sw[64 + 2 * lane + 1], db.y * xb.y);
-      da.x *= wa.x; da.y *= wa.y; db.x *= wb.x; db.y *= wb.y;
-      float dot = warp_sum(da.x * xa.x + da.y * xa.y + db.x * xb.x + db.y * xb.y) / D;
-      da.x = rs * (da.x - xa.x * dot);
-      da.y = rs * (da.y - xa.y * dot);
-      db.x = rs * (db.x - xb.x * dot);
-      db.y = rs * (db.y - xb.y * dot);
+  const int lane = threadIdx.x & 31, l = lane & 7;
+  const int heads = Hq + Hkv, all = Hq + 2 * Hkv;
+  const int groups = (all + kRopeHeads - 1) / kRopeHeads;
+  const int gw = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int walkers = static_cast<int>((gridDim.x * blockDim.x) >> 5) / groups;  // warps that share a group of heads
+  const int h = (gw % groups) * kRopeHeads + (lane >> 3);
+  const bool is_q = h < Hq, is_v = h >= heads;
+  const int hs = min(h, all - 1);
+  const __nv_bfloat16* g0 = is_q ? dq + static_cast<long long>(h) * D
+                                 : !is_v ? dk + static_cast<long long>(h - Hq) * D
+                                         : dv + static_cast<long long>(hs - heads) * D;
+  const long long gpitch = static_cast<long long>(is_q ? Hq : Hkv) * D;
+  RopeVec acc;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc.a[j] = acc.b[j] = 0.f;
+  RopeVec ww;
+  if (has_norm) ww.read(is_q ? qw : kw, l);
+  if (gw < walkers * groups)
+    for (int t = gw / groups; t < T; t += walkers) {
+      const __nv_bfloat16* g = g0 + t * gpitch;
+      const BF8 raw_a = reinterpret_cast<const BF8*>(g)[l], raw_b = reinterpret_cast<const BF8*>(g + 64)[l];
+      const long long row = static_cast<long long>(t) * all;
+      RopeVec x;
+      float rs = 0.f;
+      if (has_norm) {
+        x.read(qkv + (row + hs) * D, l);
+        rs = is_v ? 0.f : rstd[static_cast<long long>(t) * heads + h];
+      }
+      RopeAngles r;
+      r.read(cos_t, sin_t, pos[t], l);
+      RopeVec d;
+      {
+        float ga[8], gb[8];
+        bf8_to_float(raw_a, ga);
+        bf8_to_float(raw_b, gb);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // transpose of the rotation
+          d.a[j] = ga[j] * r.c[j] + gb[j] * r.s[j];
+          d.b[j] = gb[j] * r.c[j] - ga[j] * r.s[j];
+        }
+      }
+      if (has_norm) {
+        float dot = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          x.a[j] *= rs;
+          x.b[j] *= rs;
+          acc.a[j] += d.a[j] * x.a[j];
+          acc.b[j] += d.b[j] * x.b[j];
+          d.a[j] *= ww.a[j];
+          d.b[j] *= ww.b[j];
+          dot += d.a[j] * x.a[j] + d.b[j] * x.b[j];
+        }
+        dot = rope_sum8(dot) / D;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          d.a[j] = rs * (d.a[j] - x.a[j] * dot);
+          d.b[j] = rs * (d.b[j] - x.b[j] * dot);
+        }
+      }
+      if (h >= all) continue;
+      __nv_bfloat16* out = dqkv + (row + h) * D;
+      if (is_v) {
+        reinterpret_cast<BF8*>(out)[l] = raw_a;
+        reinterpret_cast<BF8*>(out + 64)[l] = raw_b;
+      } else {
+        d.write(out, l);
+      }
     }
-    reinterpret_cast<__nv_bfloat162*>(out)[lane] = __floats2bfloat162_rn(da.x, da.y);
-    reinterpret_cast<__nv_bfloat162*>(out + 64)[lane] = __floats2bfloat162_rn(db.x, db.y);
+  if (!has_norm) return;
+  if (!is_v) {
+    float* sw = s_dw[is_q ? 0 : 1];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      atomicAdd(&sw[8 * l + j], acc.a[j]);
+      atomicAdd(&sw[64 + 8 * l + j], acc.b[j]);
+    }
   }
-  if (has_norm) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-      if (s_dw[0][i] != 0.f) atomicAdd(&dqw[i], s_dw[0][i]);
-      if (s_dw[1][i] != 0.f) atomicAdd(&dkw[i], s_dw[1][i]);
-    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    if (s_dw[0][i] != 0.f) atomicAdd(&dqw[i], s_dw[0][i]);
+    if (s_dw[1][i] != 0.f) atomicAdd(&dkw[i], s_dw[1][i]);
   }
 }
 
 // ------------------------------------------------------------------- SwiGLU --
-// gu: [T, 2*I] (gate = first I columns, up = last I columns); out: [T, I].
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ out, long long T, int I) {
-  const int nvec = I >> 3;
-  const long long total = T * nvec;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long t = i / nvec;
-    const int c = static_cast<int>(i % nvec);
-    float g[8], u[8], o[8];
-    bf8_to_float(reinterpret_cast<const BF8*>(gu + t * 2 * I)[c], g);
-    bf8_to_float(reinterpret_cast<const BF8*>(gu + t * 2 * I + I)[c], u);
+// gu: [T, 2*I] (gate = first I columns, up = last I columns); out: [T, I]. A thread takes the same vector of ROWS rows
+// and loads all of them before it computes; rows and columns come from the grid, not from a 64-bit division per vector, and the
+// sigmoid is one approximate reciprocal (1 ulp; the exponential before it is no better), because IEEE divisions alone kept
+// the issue slots busy for most of the time that the memory needs. Two rows a thread; one is 4% slower, four 30%. 16384 x 6144:
+// 129 us forward and 181 us backward before, 96 and 146 us (6.3 and 6.9 TB/s) now.
+__device__ __forceinline__ float sigmoid_rcp(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-x)));
+  return r;
+}
+
+template <int ROWS>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= I >> 3) return;
+  for (long long t0 = static_cast<long long>(blockIdx.y) * ROWS; t0 < T; t0 += static_cast<long long>(gridDim.y) * ROWS) {
+    BF8 g[ROWS], u[ROWS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
-    reinterpret_cast<BF8*>(out + t * I)[c] = float_to_bf8(o);
+    for (int r = 0; r < ROWS; ++r)
+      if (t0 + r < T) {
+        g[r] = reinterpret_cast<const BF8*>(gu + (t0 + r) * 2 * I)[c];
+        u[r] = reinterpret_cast<const BF8*>(gu + (t0 + r) * 2 * I + I)[c];
+      }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+      if (t0 + r < T) {
+        float fg[8], fu[8], o[8];
+        bf8_to_float(g[r], fg);
+        bf8_to_float(u[r], fu);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = fg[j] * sigmoid_rcp(fg[j]) * fu[j];
+        reinterpret_cast<BF8*>(out + (t0 + r) * I)[c] = float_to_bf8(o);
+      }
   }
 }
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                  const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ dgu, long long T, int I) {
-  const int nvec = I >> 3;
-  const long long total = T * nvec;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long t = i / nvec;
-    const int c = static_cast<int>(i % nvec);
-    float g[8], u[8], d[8], dg[8], du[8];
-    bf8_to_float(reinterpret_cast<const BF8*>(gu + t * 2 * I)[c], g);
-    bf8_to_float(reinterpret_cast<const BF8*>(gu + t * 2 * I + I)[c], u);
-    bf8_to_float(reinterpret_cast<const BF8*>(dy + t * I)[c], d);
+template <int ROWS>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
+                  __nv_bfloat16* __restrict__ dgu, long long T, int I) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= I >> 3) return;
+  for (long long t0 = static_cast<long long>(blockIdx.y) * ROWS; t0 < T; t0 += static_cast<long long>(gridDim.y) * ROWS) {
+    BF8 g[ROWS], u[ROWS], d[ROWS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sg = 1.f / (1.f + __expf(-g[j]));
-      const float silu = g[j] * sg;
-      du[j] = d[j] * silu;
-      dg[j] = d[j] * u[j] * (sg * (1.f + g[j] * (1.f - sg)));
-    }
-    reinterpret_cast<BF8*>(dgu + t * 2 * I)[c] = float_to_bf8(dg);
-    reinterpret_cast<BF8*>(dgu + t * 2 * I + I)[c] = float_to_bf8(du);
+    for (int r = 0; r < ROWS; ++r)
+      if (t0 + r < T) {
+        g[r] = reinterpret_cast<const BF8*>(gu + (t0 + r) * 2 * I)[c];
+        u[r] = reinterpret_cast<const BF8*>(gu + (t0 + r) * 2 * I + I)[c];
+        d[r] = reinterpret_cast<const BF8*>(dy + (t0 + r) * I)[c];
+      }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+      if (t0 + r < T) {
+        float fg[8], fu[8], fd[8], dg[8], du[8];
+        bf8_to_float(g[r], fg);
+        bf8_to_float(u[r], fu);
+        bf8_to_float(d[r], fd);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float sg = sigmoid_rcp(fg[j]);
+          const float silu = fg[j] * sg;
+          du[j] = fd[j] * silu;
+          dg[j] = fd[j] * fu[j] * (sg * (1.f + fg[j] * (1.f - sg)));
+        }
+        reinterpret_cast<BF8*>(dgu + (t0 + r) * 2 * I)[c] = float_to_bf8(dg);
+        reinterpret_cast<BF8*>(dgu + (t0 + r) * 2 * I + I)[c] = float_to_bf8(du);
+      }
   }
 }
 
-template <typename F>
-static int dispatch_nv(int H, F&& f) {
-  const int nv = (H / 8 + 31) / 32;
-  if (nv <= 1) return f(std::integral_constant<int, 1>{});
-  if (nv <= 2) return f(std::integral_constant<int, 2>{});
-  if (nv <= 4) return f(std::integral_constant<int, 4>{});
-  if (nv <= 8) return f(std::integral_constant<int, 8>{});
-  if (nv <= 16) return f(std::integral_constant<int, 16>{});
-  if (nv <= 32) return f(std::integral_constant<int, 32>{});
-  return -101;
+// (columns / 256, rows / ROWS) blocks; the kernels walk on where that is more than a grid holds
+static dim3 swiglu_grid(long long T, int I, int rows, int& threads) {
+  const int nvec = I >> 3;
+  threads = nvec >= 256 ? 256 : (nvec + 31) / 32 * 32;
+  const long long y = (T + rows - 1) / rows;
+  return dim3((nvec + threads - 1) / threads, static_cast<unsigned>(y < 65535 ? y : 65535));
+}
+
+template <class F>
+static int rms_dispatch(int H, F&& f) {
+  const RmsShape s = rms_shape(H);
+  if (s.group > 512) return -101;
+  return s.vpt == 1 ? f(std::integral_constant<int, 1>{}, s.group) : f(std::integral_constant<int, 2>{}, s.group);
 }
 
 }  // namespace b200
@@ -432,12 +586,10 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   using namespace b200;
   if (T == 0) return 0;
   if (H % 8) return -100;
-  const int wpb = 4;
-  int grid = (T + wpb - 1) / wpb;
-  const int maxg = sm_count() * 16;
-  if (grid > maxg) grid = maxg;
-  int rc = dispatch_nv(H, [&](auto nv) {
-    rmsnorm_fwd_kernel<decltype(nv)::value><<<grid, wpb * 32, 0, stream>>>(
+  int rc = rms_dispatch(H, [&](auto vpt, int group) {
+    const int groups = 256 / group > 1 ? 256 / group : 1;
+    constexpr int R = 2;
+    rmsnorm_fwd_kernel<decltype(vpt)::value, R><<<(T + groups * R - 1) / (groups * R), dim3(group, groups), 0, stream>>>(
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
         (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd, T, H, eps);
     return 0;
@@ -459,21 +611,19 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
   using namespace b200;
   if (T == 0) return 0;
   if (H % 8) return -100;
-  const int wpb = 4;
   const int grid = b200_rmsnorm_bwd_blocks(T);
-  const size_t smem = static_cast<size_t>(wpb) * H * sizeof(float);
-  int rc = dispatch_nv(H, [&](auto nv) {
-    auto k = rmsnorm_bwd_kernel<decltype(nv)::value>;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<grid, wpb * 32, smem, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                                        (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
-                                        (__nv_bfloat16*)dx, dw_partial, T, H);
+  int rc = rms_dispatch(H, [&](auto vpt, int group) {
+    // 512 threads a block, two blocks an SM; at most 8 rows side by side (a named barrier each)
+    const int rows = 512 / group > 8 ? 8 : 512 / group;
+    rmsnorm_bwd_kernel<decltype(vpt)::value>
+        <<<grid, dim3(group, rows), static_cast<size_t>(rows - 1) * H * sizeof(float), stream>>>(
+            (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+            (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, T, H);
     return 0;
   });
   if (rc) return rc;
-  colsum_partials_kernel<<<(H + 255) / 256, 256, 0, stream>>>(dw_partial, dw, grid, H,
-                                                              dw_accumulate);
+  B200_CHECK(cudaGetLastError());
+  colsum_partials_kernel<<<(H + 31) / 32, 512, 0, stream>>>(dw_partial, dw, grid, H, dw_accumulate);
   B200_CHECK(cudaGetLastError());
   return 0;
 }
@@ -485,7 +635,7 @@ int b200_qknorm_rope_fwd(const void* qkv, const void* qw, const void* kw, const 
   using namespace b200;
   if (D != 128) return -100;
   if (T == 0) return 0;
-  const long long warps = static_cast<long long>(T) * (Hq + Hkv);
+  const long long warps = static_cast<long long>(T) * ((Hq + Hkv + 2 * kRopeHeads - 1) / (2 * kRopeHeads));
   const int tpb = 256;
   const long long grid = (warps * 32 + tpb - 1) / tpb;
   qknorm_rope_fwd_kernel<<<(unsigned)grid, tpb, 0, stream>>>(
@@ -504,8 +654,8 @@ int b200_qknorm_rope_kvwrite(const void* qkv, const void* qw, const void* kw, co
   using namespace b200;
   if (D != 128) return -100;
   if (T == 0) return 0;
-  const long long warps = static_cast<long long>(T) * (Hq + 2 * Hkv);
-  const int tpb = 256;
+  const long long warps = static_cast<long long>(T) * ((Hq + 2 * Hkv + kRopeHeads - 1) / kRopeHeads);
+  const int tpb = 128;
   const long long grid = (warps * 32 + tpb - 1) / tpb;
   qknorm_rope_kvwrite_kernel<<<(unsigned)grid, tpb, 0, stream>>>(
       (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cos_t, sin_t, pos,
@@ -515,19 +665,24 @@ int b200_qknorm_rope_kvwrite(const void* qkv, const void* qw, const void* kw, co
   return 0;
 }
 
-// dqw/dkw are fp32 [D] accumulators (added to, not overwritten).
-int b200_qknorm_rope_bwd(const void* dq, const void* dk, const void* qkv, const void* qw,
+// dqw/dkw are fp32 [D] accumulators (added to, not overwritten); dq [T, Hq, D], dk and dv [T, Hkv, D] contiguous.
+int b200_qknorm_rope_bwd(const void* dq, const void* dk, const void* dv, const void* qkv, const void* qw,
                          const void* kw, const float* cos_t, const float* sin_t, const int* pos,
                          const float* rstd, void* dqkv, float* dqw, float* dkw, int T, int Hq,
                          int Hkv, int D, int has_norm, cudaStream_t stream) {
   using namespace b200;
   if (D != 128) return -100;
   if (T == 0) return 0;
-  const long long warps = static_cast<long long>(T) * (Hq + Hkv);
+  const int groups = (Hq + 2 * Hkv + kRopeHeads - 1) / kRopeHeads;
+  const long long warps = static_cast<long long>(T) * groups;
   const int tpb = 256;
-  const long long grid = (warps * 32 + tpb - 1) / tpb;
+  // three blocks an SM are resident; every group of heads needs a warp of its own
+  long long grid = (warps * 32 + tpb - 1) / tpb;
+  const long long least = (groups * 32 + tpb - 1) / tpb, most = static_cast<long long>(sm_count()) * 3;
+  if (grid > most) grid = most;
+  if (grid < least) grid = least;
   qknorm_rope_bwd_kernel<<<(unsigned)grid, tpb, 0, stream>>>(
-      (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)qkv,
+      (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, (const __nv_bfloat16*)qkv,
       (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cos_t, sin_t, pos, rstd,
       (__nv_bfloat16*)dqkv, dqw, dkw, T, Hq, Hkv, has_norm);
   B200_CHECK(cudaGetLastError());
@@ -538,12 +693,9 @@ int b200_swiglu_fwd(const void* gu, void* out, long long T, int I, cudaStream_t 
   using namespace b200;
   if (T == 0) return 0;
   if (I % 8) return -100;
-  long long total = T * (I / 8);
-  long long grid = (total + 255) / 256;
-  const long long maxg = static_cast<long long>(sm_count()) * 16;
-  if (grid > maxg) grid = maxg;
-  swiglu_fwd_kernel<<<(unsigned)grid, 256, 0, stream>>>((const __nv_bfloat16*)gu,
-                                                        (__nv_bfloat16*)out, T, I);
+  int threads;
+  const dim3 grid = swiglu_grid(T, I, 2, threads);
+  swiglu_fwd_kernel<2><<<grid, threads, 0, stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I);
   B200_CHECK(cudaGetLastError());
   return 0;
 }
@@ -552,12 +704,10 @@ int b200_swiglu_bwd(const void* dy, const void* gu, void* dgu, long long T, int 
   using namespace b200;
   if (T == 0) return 0;
   if (I % 8) return -100;
-  long long total = T * (I / 8);
-  long long grid = (total + 255) / 256;
-  const long long maxg = static_cast<long long>(sm_count()) * 16;
-  if (grid > maxg) grid = maxg;
-  swiglu_bwd_kernel<<<(unsigned)grid, 256, 0, stream>>>(
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, I);
+  int threads;
+  const dim3 grid = swiglu_grid(T, I, 2, threads);
+  swiglu_bwd_kernel<2><<<grid, threads, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu,
+                                                     (__nv_bfloat16*)dgu, T, I);
   B200_CHECK(cudaGetLastError());
   return 0;
 }
@@ -604,19 +754,5 @@ extern "C" int b200_rmsnorm_bwd_static(const void* dy, const void* x, const void
     }
     scratch = g_scratch_ptr[dev];
   }
-  const int wpb = 4;
-  const size_t smem = static_cast<size_t>(wpb) * H * sizeof(float);
-  int rc = dispatch_nv(H, [&](auto nv) {
-    auto k = rmsnorm_bwd_kernel<decltype(nv)::value>;
-    if (smem > 48 * 1024)
-      B200_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, wpb * 32, smem, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                        rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, T, H);
-    B200_CHECK(cudaGetLastError());
-    return 0;
-  });
-  if (rc) return rc;
-  colsum_partials_kernel<<<(H + 255) / 256, 256, 0, stream>>>(scratch, dw, grid, H, dw_accumulate);
-  B200_CHECK(cudaGetLastError());
-  return 0;
+  return b200_rmsnorm_bwd(dy, x, w, rstd, dres, dx, scratch, dw, dw_accumulate, T, H, stream);
 }

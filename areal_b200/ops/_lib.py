@@ -79,6 +79,15 @@ def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+def vec16(t: torch.Tensor | None) -> torch.Tensor | None:
+    """``t`` contiguous on a 16-byte boundary, for kernels that read it in 16-byte vectors: a slice of a larger buffer may
+    start anywhere, and is copied where it does."""
+    if t is None:
+        return t
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise RuntimeError(f"areal_b200 native call {what} failed with code {rc}")

@@ -178,7 +178,7 @@ class _QKNormRope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps):
         T = qkv.shape[0]
-        qkv = qkv if qkv.is_contiguous() else qkv.contiguous()
+        qkv, qw, kw, cos, sin = (_lib.vec16(t) for t in (qkv, qw, kw, cos, sin))
         has_norm = qw is not None
         q = torch.empty((T, Hq, D), dtype=qkv.dtype, device=qkv.device)
         k = torch.empty((T, Hkv, D), dtype=qkv.dtype, device=qkv.device)
@@ -206,24 +206,22 @@ class _QKNormRope(torch.autograd.Function):
         qkv, qw, kw, cos, sin, pos, rstd = ctx.saved_tensors
         T, Hq, Hkv, D, has_norm = ctx.dims
         dqkv = torch.empty_like(qkv)
-        # dv goes straight into the v slot of the fused gradient
-        dqkv[:, (Hq + Hkv) * D:].view(T, Hkv, D).copy_(dv)
-        dq = dq if dq.is_contiguous() else dq.contiguous()
-        dk = dk if dk.is_contiguous() else dk.contiguous()
-        dqw = torch.zeros(D, dtype=torch.float32, device=qkv.device)
-        dkw = torch.zeros(D, dtype=torch.float32, device=qkv.device)
+        dq, dk, dv = _lib.vec16(dq), _lib.vec16(dk), _lib.vec16(dv)
+        dw = torch.zeros((2, D), dtype=torch.float32, device=qkv.device)  # of the q and the k norm
         lib = _lib.kernels()
         lib.b200_qknorm_rope_bwd.restype = ctypes.c_int
-        rc = lib.b200_qknorm_rope_bwd(_lib.ptr(dq), _lib.ptr(dk), _lib.ptr(qkv), _lib.ptr(qw),
-                                      _lib.ptr(kw), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos),
-                                      _lib.ptr(rstd), _lib.ptr(dqkv), _lib.ptr(dqw), _lib.ptr(dkw),
+        rc = lib.b200_qknorm_rope_bwd(_lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(qkv),
+                                      _lib.ptr(qw), _lib.ptr(kw), _lib.ptr(cos), _lib.ptr(sin),
+                                      _lib.ptr(pos), _lib.ptr(rstd), _lib.ptr(dqkv), _lib.ptr(dw[0]),
+                                      _lib.ptr(dw[1]),
                                       ctypes.c_int(T), ctypes.c_int(Hq), ctypes.c_int(Hkv),
                                       ctypes.c_int(D), ctypes.c_int(int(has_norm)),
                                       _lib.stream_ptr())
         _lib.check(rc, "b200_qknorm_rope_bwd")
         _lib.count_launch()
         if has_norm:
-            return dqkv, dqw.to(qw.dtype), dkw.to(kw.dtype), None, None, None, None, None, None, None
+            dqw, dkw = dw.to(qw.dtype).unbind(0)
+            return dqkv, dqw, dkw, None, None, None, None, None, None, None
         return dqkv, None, None, None, None, None, None, None, None, None
 
 
@@ -252,13 +250,15 @@ def qknorm_rope_kvwrite(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps, slot_mappin
     """Inference form of :func:`qknorm_rope`: returns ``q [T, Hq, D]`` and writes the normalised,
     rotated ``k`` and the raw ``v`` into the paged caches ``[num_blocks, Hkv, block_size, D]`` at
     ``slot_mapping [T]`` (int64, negative = skip) in the same kernel."""
-    if not (_lib.use_cuda_kernels(qkv, k_cache) and qkv.dtype == torch.bfloat16 and D == 128 and qkv.is_contiguous()):
+    if not (_lib.use_cuda_kernels(qkv, k_cache) and qkv.dtype == torch.bfloat16 and D == 128 and qkv.is_contiguous()
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0):
         from .rollout_ops import kv_cache_write
 
         q, k, v = qknorm_rope(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps)
         kv_cache_write(k, v, slot_mapping, k_cache, v_cache)
         return q
     T = qkv.shape[0]
+    qkv, qw, kw, cos, sin = (_lib.vec16(t) for t in (qkv, qw, kw, cos, sin))
     q = torch.empty((T, Hq, D), dtype=qkv.dtype, device=qkv.device)
     slots = slot_mapping if slot_mapping.dtype == torch.int64 else slot_mapping.to(torch.int64)
     if _lib.checked():
