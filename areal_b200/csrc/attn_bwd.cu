@@ -5,20 +5,26 @@
 // accumulators in TMEM (2 x 128 columns) while it walks every query block i on
 // or below the causal diagonal, for every query head of the GQA group:
 //
-//   S^T  = K_j Q_i^T            (tcgen05, TMEM cols 256..383)
-//   dP^T = V_j dO_i^T           (tcgen05, TMEM cols 384..511)
-//   P^T  = exp2(S^T*c - lse_i)  (registers → bf16 → swizzled smem)
-//   dV  += P^T dO_i             (tcgen05; dO_i read MN-major from the same tile)
-//   dS^T = P^T ∘ (dP^T - Δ_i) * scale
-//   dK  += dS^T Q_i             (tcgen05; Q_i read MN-major)
-//   dQ_i = dS K_j               (tcgen05 into the S^T columns; both operands MN-major;
-//                                then red.global.add.v4.f32 into an fp32 dQ buffer)
+//   S^T   = K_j Q_i^T           (TMEM cols 256..383)
+//   dP^T  = V_j dO_i^T          (TMEM cols 384..511)
+//   P^T   = exp2(S^T*c - lse_i) (registers → bf16 → TMEM, over the S^T columns it came from)
+//   dV   += P^T dO_i            (A operand from TMEM; dO_i read MN-major from the same tile)
+//   dS^T  = P^T ∘ (dP^T - Δ_i)  (registers → bf16 → swizzled smem; the softmax scale is applied to dK and dQ)
+//   dQ_i^T = K_j^T dS^T         (over the dP^T columns; both operands MN-major)
+//   dK   += dS^T Q_i            (Q_i read MN-major)
 //
 // Working on the transposed score tile makes each compute thread own (part of)
 // one key row, so P^T and dS^T are written row-per-thread as K-major A operands
-// and no tile is ever transposed in memory. The kernel is a template on the number
-// of compute warps: with 8, warps w and w+4 read the same 32 TMEM lanes and take
-// the lower / upper 64 columns of every 128-column tile.
+// and no tile is ever transposed in memory. dQ is produced transposed as well: a lane of
+// the warps that drain it owns a head dimension, so the 32 lanes of a reduction into the fp32 dQ buffer hit one
+// 128-byte line (with a query row per lane every lane touched a line of its own).
+//
+// What bounds it: 5 products of 128^3 take 2550 cycles per tile pair at the tensor cores' rate, their operands 2300
+// cycles of shared memory bandwidth (P^T from TMEM saves a write and a read of 32 KB), the exponentials 1024 cycles. In sequence these and
+// their hand-offs take four times as long, so the roles overlap: S^T of the next block is issued as soon as P^T is
+// consumed and is ready while the compute warps still work on dS^T; four warps of their own drain dQ while
+// dK accumulates. Before, one warp set did everything in turn: 8 sequences of 8192, 16 / 8 heads: 11.6 ms (472
+// TFLOP/s), now 6.7 ms (825 TFLOP/s).
 //
 // Replaces flash-attn's backward / aten._flash_attention_backward in the
 // reference (areal/experimental/models/archon/attention/varlen.py:116).
@@ -29,8 +35,9 @@ namespace b200 {
 
 constexpr int kD = 128;
 constexpr int kBT = 128;  // rows of every tile (q and kv)
-// NCW compute warps (4 or 8) + TMA producer + MMA issuer
-template <int NCW> constexpr int bwd_threads() { return NCW * 32 + 64; }
+constexpr int kBwdCompute = 8;  // compute warps: w and w + 4 share 32 TMEM lanes and take 64 columns each
+constexpr int kBwdDrain = 4;    // warps that take dQ out of TMEM and stage the row statistics
+constexpr int kBwdThreads = (kBwdCompute + kBwdDrain + 2) * 32;  // + TMA producer + MMA issuer
 
 struct AttnBwdTile {
   int kv_start;   // first global token row of this kv block
@@ -43,7 +50,7 @@ struct AttnBwdTile {
 };
 
 constexpr int kTileBytes = kBT * kD * 2;  // 32 KB
-// K, V resident; (Q, dO) x 2 stages; one buffer shared by P^T and dS^T.
+// K, V resident; (Q, dO) x 2 stages; dS^T.
 constexpr int kAttnBwdSmem = 2 * kTileBytes + 4 * kTileBytes + kTileBytes;  // 224 KB
 
 // Δ[h, t] = sum_d dO[t,h,d] * O[t,h,d]
@@ -81,17 +88,62 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* 
   }
 }
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c),
-               "f"(d)
-               : "memory");
+__device__ __forceinline__ void red_add(float* addr, float a) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(a) : "memory");
+}
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// D[tmem] (+)= A[tmem] * B[smem desc]: A holds two bf16 per 32-bit column, 8 columns per 16-wide reduction step
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 
-// TREE: keys carry a subtree end (`key_exit`) that bounds the queries they are visible to. It is a
-// template flag because the 4-warp variant sits at the register limit: the extra compare in the
-// innermost loop cost the ordinary causal path a third of its speed when it was a run-time test.
-template <int NCW, bool TREE>
-__global__ void __launch_bounds__(NCW * 32 + 64, 1)
+// What a compute thread needs to know to mask its key row against a query block.
+struct BwdMask {
+  bool kv_valid, diag;
+  int q0, q_rows, kv_pos, kv_exit;
+  template <bool TREE>
+  __device__ __forceinline__ bool valid(int col) const {
+    bool v = kv_valid && (col < q_rows) && (!diag || (q0 + col >= kv_pos));
+    if (TREE) v = v && (q0 + col < kv_exit);
+    return v;
+  }
+};
+
+// 32 columns of P^T: exp2(S^T * c - lse), packed to bf16.
+template <bool MASK, bool TREE>
+__device__ __forceinline__ void bwd_p32(const uint32_t (&raw)[32], const float* lse, int col0, float scale_log2,
+                                        const BwdMask& m, uint32_t* packed) {
+#pragma unroll
+  for (int e = 0; e < 32; e += 4) {
+    const float4 l = *reinterpret_cast<const float4*>(lse + e);
+    const float lv[4] = {l.x, l.y, l.z, l.w};
+    float p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      p[u] = exp2_ftz(__uint_as_float(raw[e + u]) * scale_log2 - lv[u]);
+      if (MASK) p[u] = m.valid<TREE>(col0 + e + u) ? p[u] : 0.f;
+    }
+    __nv_bfloat162 a = __floats2bfloat162_rn(p[0], p[1]), b = __floats2bfloat162_rn(p[2], p[3]);
+    packed[e / 2] = *reinterpret_cast<uint32_t*>(&a);
+    packed[e / 2 + 1] = *reinterpret_cast<uint32_t*>(&b);
+  }
+}
+
+// TREE: keys carry a subtree end (`key_exit`) that bounds the queries they are visible to.
+template <bool TREE>
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const AttnBwdTile* __restrict__ tiles, const float* __restrict__ lse,
@@ -99,32 +151,33 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, int T, int Hq,
                 int Hkv, long long lddk, long long lddv, float scale, int* status,
                 const int* __restrict__ key_exit) {
-  constexpr int kCompute = NCW * 32;     // compute threads
-  constexpr int kChunks = 4 / (NCW / 4);  // 32-column chunks of a 128-column tile per compute warp
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ uint64_t bars[16];
+  __shared__ uint64_t bars[20];
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_word;
-  __shared__ float s_lse[2][kBT];
-  __shared__ float s_delta[2][kBT];
+  __shared__ __align__(16) float s_lse[2][kBT];
+  __shared__ __align__(16) float s_delta[2][kBT];
   volatile int* abort_flag = &abort_word;
 
   uint8_t* sK = smem;
   uint8_t* sV = smem + kTileBytes;
   uint8_t* sQ = smem + 2 * kTileBytes;   // [2 stages]
   uint8_t* sdO = smem + 4 * kTileBytes;  // [2 stages]
-  uint8_t* sPS = smem + 6 * kTileBytes;  // P^T, then dS^T
+  uint8_t* sdS = smem + 6 * kTileBytes;  // dS^T
   uint64_t* kv_full = &bars[0];
-  uint64_t* qdo_full = &bars[1];   // [2]
-  uint64_t* qdo_empty = &bars[3];  // [2]
-  uint64_t* s_full = &bars[5];
-  uint64_t* dp_full = &bars[6];
-  uint64_t* pt_ready = &bars[7];
-  uint64_t* pbuf_free = &bars[8];
-  uint64_t* dst_ready = &bars[9];
-  uint64_t* dq_full = &bars[10];
-  uint64_t* dq_read = &bars[11];
-  uint64_t* acc_done = &bars[12];
+  uint64_t* q_full = &bars[1];    // [2]
+  uint64_t* q_empty = &bars[3];   // [2]
+  uint64_t* do_full = &bars[5];   // [2]
+  uint64_t* do_empty = &bars[7];  // [2]
+  uint64_t* ls_full = &bars[9];   // [2] lse and delta of a block are staged
+  uint64_t* s_full = &bars[11];
+  uint64_t* dp_full = &bars[12];
+  uint64_t* p_ready = &bars[13];
+  uint64_t* ds_ready = &bars[14];
+  uint64_t* ds_free = &bars[15];  // the products that read dS^T are done
+  uint64_t* dq_full = &bars[16];
+  uint64_t* dq_read = &bars[17];
+  uint64_t* acc_done = &bars[18];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -136,7 +189,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   // (context parallelism: this rank owns the positions [q_begin, seq_len) of the sequence)
   const int qb_first = max(tile.kv_off, tile.q_begin) / kBT;
   const int qb_count = (tile.seq_len + kBT - 1) / kBT - qb_first;
-  const int n_iter = qb_count * group;  // iteration it -> (head g = it / qb_count, block i = it % qb_count)
+  const int n_iter = qb_count > 0 ? qb_count * group : 0;  // iteration it -> (head g = it / qb_count, block i = it % qb_count)
   const float scale_log2 = scale * 1.4426950408889634f;
 
   if (threadIdx.x == 0) {
@@ -144,16 +197,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (abort_word) atomicCAS(status, 0, kErrBounds);
     mbar_init(kv_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&do_full[i], 1);
+      mbar_init(&do_empty[i], 1);
+      mbar_init(&ls_full[i], kBwdDrain * 32);
     }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(pt_ready, kCompute);
-    mbar_init(pbuf_free, 1);
-    mbar_init(dst_ready, kCompute);
+    mbar_init(p_ready, kBwdCompute * 32);
+    mbar_init(ds_ready, kBwdCompute * 32);
+    mbar_init(ds_free, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_read, kCompute);
+    mbar_init(dq_read, kBwdDrain * 32);
     mbar_init(acc_done, 1);
     fence_mbar_init();
     prefetch_tmap(&tmQ);
@@ -161,7 +217,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     prefetch_tmap(&tmV);
     prefetch_tmap(&tmdO);
   }
-  if (warp == NCW + 1) {
+  constexpr int kTmaWarp = kBwdCompute + kBwdDrain, kMmaWarp = kTmaWarp + 1;
+  if (warp == kMmaWarp) {
     tmem_alloc(&tmem_holder, 512);
     tmem_relinquish();
   }
@@ -171,12 +228,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tmem_base = tmem_holder;
   const uint32_t tm_dK = tmem_base;
   const uint32_t tm_dV = tmem_base + 128;
-  const uint32_t tm_S = tmem_base + 256;   // S^T, later dQ
-  const uint32_t tm_dP = tmem_base + 384;  // dP^T
+  const uint32_t tm_S = tmem_base + 256;   // S^T, then P^T (its first and its third quarter)
+  const uint32_t tm_dP = tmem_base + 384;  // dP^T, then dQ^T
   const bool bad_align = (abort_word != 0);
 
   if (bad_align) {
-  } else if (warp == NCW) {
+  } else if (warp == kTmaWarp) {
     // ------------------------------------------------------ TMA producer --
     if (elect_one_sync()) {
       mbar_arrive_expect_tx(kv_full, 2 * kTileBytes);
@@ -191,12 +248,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int g = it / qb_count, i = qb_first + it % qb_count;
         const int h = hk * group + g;
         const int row = tile.seq_start + i * kBT;
-        if (!mbar_wait(&qdo_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
-        mbar_arrive_expect_tx(&qdo_full[st], 2 * kTileBytes);
-        tma_load_2d(sQ + st * kTileBytes, &tmQ, &qdo_full[st], h * kD, row);
-        tma_load_2d(sQ + st * kTileBytes + kTileBytes / 2, &tmQ, &qdo_full[st], h * kD + 64, row);
-        tma_load_2d(sdO + st * kTileBytes, &tmdO, &qdo_full[st], h * kD, row);
-        tma_load_2d(sdO + st * kTileBytes + kTileBytes / 2, &tmdO, &qdo_full[st], h * kD + 64, row);
+        if (!mbar_wait(&q_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
+        mbar_arrive_expect_tx(&q_full[st], kTileBytes);
+        tma_load_2d(sQ + st * kTileBytes, &tmQ, &q_full[st], h * kD, row);
+        tma_load_2d(sQ + st * kTileBytes + kTileBytes / 2, &tmQ, &q_full[st], h * kD + 64, row);
+        if (!mbar_wait(&do_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
+        mbar_arrive_expect_tx(&do_full[st], kTileBytes);
+        tma_load_2d(sdO + st * kTileBytes, &tmdO, &do_full[st], h * kD, row);
+        tma_load_2d(sdO + st * kTileBytes + kTileBytes / 2, &tmdO, &do_full[st], h * kD + 64, row);
       }
       if (!ok) {
         *abort_flag = 1;
@@ -205,7 +264,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
       }
     }
-  } else if (warp == NCW + 1) {
+  } else if (warp == kMmaWarp) {
     // -------------------------------------------------------- MMA issuer --
     if (elect_one_sync()) {
       // all tiles are [128 rows][2 halves of 64 columns], 128B-swizzled.
@@ -215,60 +274,76 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       //   k-step k (16 rows): base + k*2048, LBO 16K (next 64 columns), SBO 1024
       constexpr uint32_t id_kk = make_idesc(1, 1, 0, 0, kBT, kBT);  // A K-major, B K-major
       constexpr uint32_t id_kmn = make_idesc(1, 1, 0, 1, kBT, kD);  // A K-major, B MN-major
-      constexpr uint32_t id_mnmn = make_idesc(1, 1, 1, 1, kBT, kD); // both MN-major
+      constexpr uint32_t id_mnmn = make_idesc(1, 1, 1, 1, kD, kBT); // both MN-major
       constexpr uint32_t HALF = kTileBytes / 2;
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ps_addr = smem_u32(sPS);
+      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sdS);
+      // D[128 keys, 128 queries] = tile (K-major) * rows of stage (K-major)^T
+      auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
+#pragma unroll
+        for (int k = 0; k < kD / 16; ++k) {
+          const uint32_t off = (k >> 2) * HALF + (k & 3) * 32;
+          umma_f16(d, make_sdesc_sw128(a + off, 16, 1024), make_sdesc_sw128(b + off, 16, 1024), id_kk, k > 0 ? 1u : 0u);
+        }
+      };
       bool ok = mbar_wait(kv_full, 0, abort_flag);
+      if (ok && n_iter > 0) {
+        ok = mbar_wait(&q_full[0], 0, abort_flag);
+        tc_fence_after();
+        if (ok) {
+          scores(tm_S, k_addr, smem_u32(sQ));
+          umma_commit(s_full);
+          ok = mbar_wait(&do_full[0], 0, abort_flag);
+          tc_fence_after();
+        }
+        if (ok) {
+          scores(tm_dP, v_addr, smem_u32(sdO));
+          umma_commit(dp_full);
+        }
+      }
       for (int it = 0; it < n_iter && ok; ++it) {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
+        const int st = it & 1, nst = st ^ 1;
+        const uint32_t nph = ((it + 1) >> 1) & 1;
         const uint32_t itp = it & 1;
+        const bool more = it + 1 < n_iter;
         const uint32_t q_addr = smem_u32(sQ + st * kTileBytes);
         const uint32_t do_addr = smem_u32(sdO + st * kTileBytes);
-        if (!mbar_wait(&qdo_full[st], ph, abort_flag)) { ok = false; break; }
-        // the S^T columns hold dQ of the previous iteration until it has been read out
-        if (it > 0 && !mbar_wait(dq_read, (it - 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(p_ready, itp, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < kD / 16; ++k) {  // S^T = K Q^T
-          const uint32_t off = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(tm_S, make_sdesc_sw128(k_addr + off, 16, 1024),
-                   make_sdesc_sw128(q_addr + off, 16, 1024), id_kk, k > 0 ? 1u : 0u);
+        for (int k = 0; k < kBT / 16; ++k)  // dV += P^T dO   (reduction over q rows)
+          umma_f16_ts(tm_dV, tm_S + (k >> 2) * 64 + (k & 3) * 8, make_sdesc_sw128(do_addr + k * 2048, HALF, 1024), id_kmn,
+                      (it > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&do_empty[st]);
+        if (more) {
+          // products run in the order of issue: S^T of the next block overwrites P^T when dV has read it
+          if (!mbar_wait(&q_full[nst], nph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          scores(tm_S, k_addr, smem_u32(sQ + nst * kTileBytes));
+          umma_commit(s_full);
         }
-        umma_commit(s_full);
-#pragma unroll
-        for (int k = 0; k < kD / 16; ++k) {  // dP^T = V dO^T
-          const uint32_t off = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(tm_dP, make_sdesc_sw128(v_addr + off, 16, 1024),
-                   make_sdesc_sw128(do_addr + off, 16, 1024), id_kk, k > 0 ? 1u : 0u);
-        }
-        umma_commit(dp_full);
-        if (!mbar_wait(pt_ready, itp, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(ds_ready, itp, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < kBT / 16; ++k) {  // dV += P^T dO   (reduction over q rows)
-          const uint32_t aoff = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(tm_dV, make_sdesc_sw128(ps_addr + aoff, 16, 1024),
-                   make_sdesc_sw128(do_addr + k * 2048, HALF, 1024), id_kmn,
-                   (it > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(pbuf_free);
-        if (!mbar_wait(dst_ready, itp, abort_flag)) { ok = false; break; }
-        tc_fence_after();
+        for (int k = 0; k < kBT / 16; ++k)  // dQ^T = K^T dS^T  (reduction over kv rows)
+          umma_f16(tm_dP, make_sdesc_sw128(k_addr + k * 2048, HALF, 1024), make_sdesc_sw128(ds_addr + k * 2048, HALF, 1024),
+                   id_mnmn, k > 0 ? 1u : 0u);
+        umma_commit(dq_full);
 #pragma unroll
         for (int k = 0; k < kBT / 16; ++k) {  // dK += dS^T Q
           const uint32_t aoff = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(tm_dK, make_sdesc_sw128(ps_addr + aoff, 16, 1024),
-                   make_sdesc_sw128(q_addr + k * 2048, HALF, 1024), id_kmn,
+          umma_f16(tm_dK, make_sdesc_sw128(ds_addr + aoff, 16, 1024), make_sdesc_sw128(q_addr + k * 2048, HALF, 1024), id_kmn,
                    (it > 0 || k > 0) ? 1u : 0u);
         }
-#pragma unroll
-        for (int k = 0; k < kBT / 16; ++k) {  // dQ = dS K  (reduction over kv rows)
-          umma_f16(tm_S, make_sdesc_sw128(ps_addr + k * 2048, HALF, 1024),
-                   make_sdesc_sw128(k_addr + k * 2048, HALF, 1024), id_mnmn, k > 0 ? 1u : 0u);
+        umma_commit(&q_empty[st]);
+        umma_commit(ds_free);
+        if (more) {
+          if (!mbar_wait(&do_full[nst], nph, abort_flag)) { ok = false; break; }
+          // the dP^T columns hold dQ^T until it has been read out
+          if (!mbar_wait(dq_read, itp, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          scores(tm_dP, v_addr, smem_u32(sdO + nst * kTileBytes));
+          umma_commit(dp_full);
         }
-        umma_commit(&qdo_empty[st]);
-        umma_commit(dq_full);
       }
       if (ok) umma_commit(acc_done);
       if (!ok) {
@@ -276,129 +351,127 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         atomicCAS(status, 0, kErrMbarTimeoutMma);
       }
     }
+  } else if (warp >= kBwdCompute) {
+    // ------------------------------------- row statistics in, dQ^T out --
+    const int d = (warp - kBwdCompute) * 32 + lane;  // TMEM lane: a head dimension of dQ^T, a query row of the statistics
+    const uint32_t lane_addr = static_cast<uint32_t>((warp - kBwdCompute) * 32) << 16;
+    auto stage = [&](int it) {  // log2 units for lse; rows past the sequence: probability zero
+      const int g = it / qb_count, i = qb_first + it % qb_count;
+      const int h = hk * group + g;
+      const int qi = i * kBT + d;
+      const long long idx = static_cast<long long>(h) * T + tile.seq_start + qi;
+      const bool v = qi < tile.seq_len;
+      s_lse[it & 1][d] = v ? lse[idx] * 1.4426950408889634f : INFINITY;
+      s_delta[it & 1][d] = v ? delta[idx] : 0.f;
+      mbar_arrive(&ls_full[it & 1]);
+    };
+    bool ok = true;
+    if (n_iter > 0) stage(0);
+    for (int it = 0; it < n_iter && ok; ++it) {
+      // dQ of block it - 1 was complete, so the compute warps are done with the buffer of it - 1
+      if (it + 1 < n_iter) stage(it + 1);
+      const int g = it / qb_count, i = qb_first + it % qb_count;
+      const int h = hk * group + g;
+      const int q0 = i * kBT;
+      const int q_rows = min(kBT, tile.seq_len - q0);
+      float* dst = dq_acc + (static_cast<long long>(tile.seq_start + q0) * Hq + h) * kD + d;
+      const long long pitch = static_cast<long long>(Hq) * kD;
+      if (!mbar_wait(dq_full, it & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < kBT; c += 64) {
+        uint32_t raw[2][32];
+        tmem_ld_32x32(tm_dP + lane_addr + c, raw[0]);
+        tmem_ld_32x32(tm_dP + lane_addr + c + 32, raw[1]);
+        tmem_ld_wait();
+        if (c) {
+          tc_fence_before();
+          mbar_arrive(dq_read);
+        }
+        if (q_rows == kBT) {
+#pragma unroll
+          for (int e = 0; e < 64; ++e) red_add(dst + (c + e) * pitch, __uint_as_float(raw[e >> 5][e & 31]) * scale);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 64; ++e)
+            if (c + e < q_rows) red_add(dst + (c + e) * pitch, __uint_as_float(raw[e >> 5][e & 31]) * scale);
+        }
+      }
+    }
+    if (!ok && lane == 0) {
+      *abort_flag = 1;
+      atomicCAS(status, 0, kErrMbarTimeoutEpilogue);
+    }
   } else {
     // ---------------------------------------------------- compute warps --
     const int quad = warp & 3;    // TMEM lane quarter this warp may read
-    const int cpart = warp >> 2;  // which part of the columns of every 128-column tile this warp handles
-    const int r = quad * 32 + lane;  // kv row inside the block == TMEM lane (q row for dQ)
+    const int cpart = warp >> 2;  // which 64 columns of every 128-column tile this warp handles
+    const int r = quad * 32 + lane;  // kv row inside the block == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const int kv_pos = tile.kv_off + r;
-    const bool kv_valid = r < tile.kv_len;
+    const uint32_t my_S = tm_S + lane_addr + cpart * 64, my_dP = tm_dP + lane_addr + cpart * 64;
+    BwdMask m;
+    m.kv_pos = tile.kv_off + r;
+    m.kv_valid = r < tile.kv_len;
     // tree attention: this key is visible to the queries of its own subtree only
-    const int kv_exit = (TREE && kv_valid) ? key_exit[tile.kv_start + r] : 0x7fffffff;
-    uint8_t* psrow = sPS + r * 128;
+    m.kv_exit = (TREE && m.kv_valid) ? key_exit[tile.kv_start + r] : 0x7fffffff;
+    uint8_t* dsrow = sdS + cpart * (kTileBytes / 2) + r * 128;
     bool ok = true;
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t itp = it & 1;
-      const int g = it / qb_count, i = qb_first + it % qb_count;
-      const int h = hk * group + g;
-      const int q0 = i * kBT;  // offset of the q block inside the sequence
-      const int q_rows = min(kBT, tile.seq_len - q0);
-      // stage lse / delta of this q block (log2 units for lse)
-      if (cpart == 0) {
-        const int qi = q0 + r;
-        const long long idx = static_cast<long long>(h) * T + tile.seq_start + qi;
-        const bool v = r < q_rows;
-        s_lse[itp][r] = v ? lse[idx] * 1.4426950408889634f : INFINITY;
-        s_delta[itp][r] = v ? delta[idx] : 0.f;
-      }
-      named_bar_sync(1, kCompute);
+      const int i = qb_first + it % qb_count;
+      m.q0 = i * kBT;  // offset of the q block inside the sequence
+      m.q_rows = min(kBT, tile.seq_len - m.q0);
+      m.diag = m.q0 < tile.kv_off + kBT;  // block touches the causal diagonal
+      // whole blocks need no masks: the row statistics and every key row are in range
+      const bool mask = TREE || m.diag || m.q_rows < kBT || tile.kv_len < kBT;
+      if (!mbar_wait(&ls_full[itp], (it >> 1) & 1, abort_flag)) { ok = false; break; }
       if (!mbar_wait(s_full, itp, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      uint32_t p_packed[kChunks * 16];  // this warp's columns
-      const bool diag = (q0 < tile.kv_off + kBT);  // block touches the causal diagonal
+      uint32_t p[32];  // this thread's 64 columns, two to a word
 #pragma unroll
-      for (int cl = 0; cl < kChunks; ++cl) {
-        const int c = cpart * kChunks + cl;
+      for (int cl = 0; cl < 2; ++cl) {
         uint32_t raw[32];
-        tmem_ld_32x32(tm_S + lane_addr + c * 32, raw);
+        tmem_ld_32x32(my_S + cl * 32, raw);
         tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          float p2[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int col = c * 32 + 2 * e + u;  // q row inside block
-            float p = exp2f(__uint_as_float(raw[2 * e + u]) * scale_log2 - s_lse[itp][col]);
-            bool valid = kv_valid && (col < q_rows) && (!diag || (q0 + col >= kv_pos));
-            if (TREE) valid = valid && (q0 + col < kv_exit);
-            p2[u] = valid ? p : 0.f;
-          }
-          __nv_bfloat162 pb = __floats2bfloat162_rn(p2[0], p2[1]);
-          p_packed[cl * 16 + e] = *reinterpret_cast<uint32_t*>(&pb);
-        }
+        const int col = cpart * 64 + cl * 32;
+        if (mask) bwd_p32<true, TREE>(raw, &s_lse[itp][col], col, scale_log2, m, p + cl * 16);
+        else bwd_p32<false, TREE>(raw, &s_lse[itp][col], col, scale_log2, m, p + cl * 16);
       }
-      // the buffer still holds dS^T of the previous iteration until dK/dQ MMAs finished
-      if (it > 0) {
-        if (!mbar_wait(dq_full, (it - 1) & 1, abort_flag)) { ok = false; break; }
-      }
-#pragma unroll
-      for (int cp = 0; cp < kChunks * 4; ++cp) {  // 16-byte pieces of this warp's part of the row
-        uint4 pk = make_uint4(p_packed[cp * 4], p_packed[cp * 4 + 1], p_packed[cp * 4 + 2],
-                              p_packed[cp * 4 + 3]);
-        const int c = cpart * kChunks * 4 + cp;
-        const int half = c >> 3, cc = c & 7;
-        *reinterpret_cast<uint4*>(psrow + half * (kTileBytes / 2) + ((cc ^ (r & 7)) << 4)) = pk;
-      }
-      fence_proxy_async_smem();
-      mbar_arrive(pt_ready);
-      // read dQ of the previous iteration out of the S^T columns?  No: S^T of this
-      // iteration was only issued after dq_read(it-1), so dQ(it-1) is already drained.
+      tmem_st_32x32(my_S, p);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(p_ready);
       if (!mbar_wait(dp_full, itp, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      uint32_t ds_packed[kChunks * 16];
+      // the buffer holds dS^T of the previous block until dQ and dK have read it
+      if (it > 0 && !mbar_wait(ds_free, itp ^ 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-      for (int cl = 0; cl < kChunks; ++cl) {
-        const int c = cpart * kChunks + cl;
+      for (int cl = 0; cl < 2; ++cl) {
         uint32_t raw[32];
-        tmem_ld_32x32(tm_dP + lane_addr + c * 32, raw);
+        tmem_ld_32x32(my_dP + cl * 32, raw);
         tmem_ld_wait();
+        const float* dl = &s_delta[itp][cpart * 64 + cl * 32];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const __nv_bfloat162 pb = *reinterpret_cast<__nv_bfloat162*>(&p_packed[cl * 16 + e]);
-          const float2 p = __bfloat1622float2(pb);
-          const int col = c * 32 + 2 * e;
-          const float d0 = p.x * (__uint_as_float(raw[2 * e]) - s_delta[itp][col]) * scale;
-          const float d1 = p.y * (__uint_as_float(raw[2 * e + 1]) - s_delta[itp][col + 1]) * scale;
-          __nv_bfloat162 db = __floats2bfloat162_rn(d0, d1);
-          ds_packed[cl * 16 + e] = *reinterpret_cast<uint32_t*>(&db);
+        for (int e = 0; e < 32; e += 8) {  // a 16-byte piece of the row
+          const float4 d0 = *reinterpret_cast<const float4*>(dl + e), d1 = *reinterpret_cast<const float4*>(dl + e + 4);
+          const float dd[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+          uint4 out;
+          uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t w = p[cl * 16 + e / 2 + u];
+            const float pa = __uint_as_float(w << 16), pb = __uint_as_float(w & 0xffff0000u);
+            __nv_bfloat162 b = __floats2bfloat162_rn(pa * (__uint_as_float(raw[e + 2 * u]) - dd[2 * u]),
+                                                     pb * (__uint_as_float(raw[e + 2 * u + 1]) - dd[2 * u + 1]));
+            o[u] = *reinterpret_cast<uint32_t*>(&b);
+          }
+          const int piece = cl * 4 + e / 8;
+          *reinterpret_cast<uint4*>(dsrow + ((piece ^ (r & 7)) << 4)) = out;
         }
-      }
-      if (!mbar_wait(pbuf_free, itp, abort_flag)) { ok = false; break; }
-#pragma unroll
-      for (int cp = 0; cp < kChunks * 4; ++cp) {
-        uint4 pk = make_uint4(ds_packed[cp * 4], ds_packed[cp * 4 + 1], ds_packed[cp * 4 + 2],
-                              ds_packed[cp * 4 + 3]);
-        const int c = cpart * kChunks * 4 + cp;
-        const int half = c >> 3, cc = c & 7;
-        *reinterpret_cast<uint4*>(psrow + half * (kTileBytes / 2) + ((cc ^ (r & 7)) << 4)) = pk;
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(dst_ready);
-      // dQ_i: lane r is now query row q0 + r
-      if (!mbar_wait(dq_full, itp, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      {
-        const bool qv = r < q_rows;
-        float* dq_row = dq_acc + (static_cast<long long>(tile.seq_start + q0 + r) * Hq + h) * kD;
-#pragma unroll 1
-        for (int cl = 0; cl < kChunks; ++cl) {
-          const int c = cpart * kChunks + cl;
-          uint32_t raw[32];
-          tmem_ld_32x32(tm_S + lane_addr + c * 32, raw);
-          tmem_ld_wait();
-          if (qv) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              red_add_v4(dq_row + c * 32 + e * 4, __uint_as_float(raw[4 * e]),
-                         __uint_as_float(raw[4 * e + 1]), __uint_as_float(raw[4 * e + 2]),
-                         __uint_as_float(raw[4 * e + 3]));
-          }
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(dq_read);
+      mbar_arrive(ds_ready);
     }
     // epilogue: dK, dV
     if (ok) ok = mbar_wait(acc_done, 0, abort_flag);
@@ -410,9 +483,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int which = 0; which < 2; ++which) {
         __nv_bfloat16* dst = which ? dv_row : dk_row;
         const uint32_t tm = which ? tm_dV : tm_dK;
+        const float f = which ? 1.f : scale;
 #pragma unroll 1
-        for (int cl = 0; cl < kChunks; ++cl) {
-          const int c = cpart * kChunks + cl;
+        for (int cl = 0; cl < 2; ++cl) {
+          const int c = cpart * 2 + cl;
           uint32_t raw[32];
           if (n_iter > 0) {
             tmem_ld_32x32(tm + lane_addr + c * 32, raw);
@@ -421,15 +495,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
             for (int e = 0; e < 32; ++e) raw[e] = 0;
           }
-          if (kv_valid) {
+          if (m.kv_valid) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               uint4 pk;
               __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
               for (int u = 0; u < 4; ++u)
-                pb[u] = __floats2bfloat162_rn(__uint_as_float(raw[e * 8 + 2 * u]),
-                                              __uint_as_float(raw[e * 8 + 2 * u + 1]));
+                pb[u] = __floats2bfloat162_rn(__uint_as_float(raw[e * 8 + 2 * u]) * f,
+                                              __uint_as_float(raw[e * 8 + 2 * u + 1]) * f);
               reinterpret_cast<uint4*>(dst + c * 32)[e] = pk;
             }
           }
@@ -443,7 +517,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
-  if (warp == NCW + 1) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -501,36 +575,18 @@ int b200_attn_bwd_ex(const void* q, const void* k, const void* v, const void* o,
                     kBT, 64);
   if (rc) return rc;
   static bool attr_set = false;
-  static int compute_warps = 8;
   if (!attr_set) {
-    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kAttnBwdSmem));
-    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kAttnBwdSmem));
-    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kAttnBwdSmem));
-    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kAttnBwdSmem));
-    // 8 compute warps by default (measured 472 vs 403 TFLOP/s); AREAL_B200_ATTN_BWD_WARPS=4 selects the
-    // variant in which one warp handles all 128 columns of its rows
-    const char* e = getenv("AREAL_B200_ATTN_BWD_WARPS");
-    if (e && atoi(e) == 4) compute_warps = 4;
+    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnBwdSmem));
+    B200_CHECK(cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnBwdSmem));
     attr_set = true;
   }
   int* status = device_status_word();
   if (!status) return -3;
   dim3 grid(n_tiles, Hkv);
-#define B200_ATTN_BWD_LAUNCH(NCW, TREE)                                                                   \
-  attn_bwd_kernel<NCW, TREE><<<grid, bwd_threads<NCW>(), kAttnBwdSmem, stream>>>(                         \
-      tmQ, tmK, tmV, tmdO, reinterpret_cast<const AttnBwdTile*>(tiles), lse, delta_ws, dq_acc,            \
-      (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, T, Hq, Hkv, lddk, lddv, softmax_scale, status, key_exit)
-  const bool tree = key_exit != nullptr;
-  if (compute_warps == 8) {
-    if (tree) B200_ATTN_BWD_LAUNCH(8, true); else B200_ATTN_BWD_LAUNCH(8, false);
-  } else {
-    if (tree) B200_ATTN_BWD_LAUNCH(4, true); else B200_ATTN_BWD_LAUNCH(4, false);
-  }
-#undef B200_ATTN_BWD_LAUNCH
+  auto kernel = key_exit ? attn_bwd_kernel<true> : attn_bwd_kernel<false>;
+  kernel<<<grid, kBwdThreads, kAttnBwdSmem, stream>>>(
+      tmQ, tmK, tmV, tmdO, reinterpret_cast<const AttnBwdTile*>(tiles), lse, delta_ws, dq_acc, (__nv_bfloat16*)dk,
+      (__nv_bfloat16*)dv, T, Hq, Hkv, lddk, lddv, softmax_scale, status, key_exit);
   B200_CHECK(cudaGetLastError());
   if (dq) {
     const long long n = static_cast<long long>(T) * Hq * kD;
