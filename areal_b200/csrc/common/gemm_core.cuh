@@ -39,7 +39,8 @@ constexpr int kGemmThreads = 192;
 
 template <int BN>
 struct GemmCfg {
-  static constexpr int kStages = (BN == 256) ? 4 : 6;
+  // 32- and 64-wide tiles are for products that stream a weight past a few rows: more stages, the same bytes in flight
+  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : BN == 64 ? 8 : 9;
   static constexpr int kABytes = kBM * kBK * 2;
   static constexpr int kBBytes = BN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
@@ -85,6 +86,11 @@ template <class E> __device__ __forceinline__ auto epi_k_load(const E& e, int m,
     -> decltype(e.k_load(m, kb, ax, ay, bx, ab, st)) { return e.k_load(m, kb, ax, ay, bx, ab, st); }
 template <class E> __device__ __forceinline__ bool epi_k_load(const E&, int, int, int&, int&, int&, volatile int*, int*,
                                                               long) { return true; }
+
+// kChained: a policy whose A operand is a weight that the kernel before this one does not write. Launched as a programmatic
+// dependent, the producer fills the pipeline's A halves ahead of the wait and B follows behind it. (K-major operands, no k_load.)
+template <class E> __device__ constexpr auto epi_chained(int) -> decltype(E::kChained) { return E::kChained; }
+template <class E> __device__ constexpr bool epi_chained(long) { return false; }
 
 template <int BN, bool A_MN, bool B_MN, class Epi>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -140,6 +146,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int ahead = 0;  // stages whose A half is under way
+      if constexpr (epi_chained<Epi>(0)) {
+        for (int it = 0, m_blk, n_blk; ahead < STAGES; ++it) {
+          if (!epi.tile(blockIdx.x, gridDim.x, it, tiles_m, tiles_n, m_blk, n_blk)) break;
+          const int kbn = epi_k_blocks(epi, m_blk, kblocks, 0);
+          for (int kb = 0; kb < kbn && ahead < STAGES; ++kb, ++ahead) {
+            mbar_arrive_expect_tx(&full[ahead], Cfg::kStageBytes);
+            tma_load_2d(smem_a + ahead * Cfg::kABytes, &tmA, &full[ahead], epi_k_begin(epi, m_blk, 0) + kb * kBK,
+                        epi_a_m0(epi, m_blk, 0));
+          }
+        }
+        pdl_wait();
+        pdl_trigger();
+      }
       for (int it = 0; ok; ++it) {
         int m_blk, n_blk;
         if (!epi.tile(blockIdx.x, gridDim.x, it, tiles_m, tiles_n, m_blk, n_blk)) break;
@@ -158,18 +178,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             ok = false;
             break;
           }
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
-            ok = false;
-            break;
+          const bool has_a = ahead > 0;
+          if (has_a) {
+            --ahead;
+          } else {
+            if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(&full[stage], Cfg::kStageBytes);
           }
-          mbar_arrive_expect_tx(&full[stage], Cfg::kStageBytes);
           uint8_t* a_dst = smem_a + stage * Cfg::kABytes;
           uint8_t* b_dst = smem_b + stage * Cfg::kBBytes;
           if (A_MN) {
 #pragma unroll
             for (int j = 0; j < kBM / 64; ++j)
               tma_load_2d(a_dst + j * 8192, &tmA, &full[stage], a_m0 + j * 64, k0 + kb * kBK);
-          } else {
+          } else if (!has_a) {
             tma_load_2d(a_dst, &tmA, &full[stage], ax, ay);
           }
           if (B_MN) {

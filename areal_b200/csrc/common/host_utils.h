@@ -96,6 +96,24 @@ inline int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType 
 // expires; the host reads it with b200_read_status().
 int* device_status_word();
 
+// Launch; with `chained`, as a programmatic dependent of the kernel before it in the stream (see pdl_wait). The caller
+// answers for that kernel: it writes nothing that this one reads ahead of its wait.
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool chained,
+                          A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline int sm_count() {
   static int n = 0;
   if (!n) {

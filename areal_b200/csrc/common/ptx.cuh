@@ -257,6 +257,13 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_
   return d;
 }
 
+// Programmatic dependent launch. A kernel that was launched as a dependent may start while the kernel before it in
+// the stream still runs: everything ahead of `pdl_wait` must touch nothing that kernel writes, and write nothing it reads.
+// Kernels here signal (`pdl_trigger`) only behind their own wait, so when a dependent starts, all kernels but the one
+// directly in front of it are complete. Launched the ordinary way both do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

@@ -10,9 +10,11 @@
 // Replaces the cuBLAS calls behind nn.Linear in the reference
 // (areal/experimental/models/archon/qwen3/model/model.py:103-293).
 #include "common/gemm_core.cuh"
+#include "common/gemm_pair.cuh"
 #include "common/host_utils.h"
 #include "common/io.cuh"
 #include "common/rms_row.cuh"
+#include "common/sigmoid.cuh"
 
 namespace b200 {
 
@@ -154,6 +156,22 @@ static int launch(const void* A, const void* B, void* C, const void* bias, int M
   return 0;
 }
 
+
+// The same product on pairs of SMs (gemm_pair.cuh).
+template <bool A_MN, bool B_MN>
+static int launch_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
+                       long long lda, long long ldb, long long ldc, int out_fp32, int accumulate,
+                       cudaStream_t stream) {
+  CUtensorMap tmA, tmB;
+  int rc = A_MN ? make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, lda * 2, 64, 64)
+                : make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda * 2, kBM, 64);
+  if (rc) return rc;
+  rc = B_MN ? make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb * 2, 64, 64)
+            : make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb * 2, PairCfg::kBN / 2, 64);
+  if (rc) return rc;
+  const StoreEpi epi{C, reinterpret_cast<const __nv_bfloat16*>(bias), ldc, M, N, out_fp32, accumulate};
+  return launch_pair_epi<A_MN, B_MN>(tmA, tmB, M, N, K, epi, stream);
+}
 
 // ---------------------------------------------------------------- grouped (per-expert) GEMMs --
 // Rows live in the padded, expert-sorted layout produced by the MoE sort: tile vm (128 rows)
@@ -311,36 +329,47 @@ static int launch_grouped(const void* A, const void* B, void* C, const int* tile
 
 
 // ------------------------------------------------------------------------------ split-K --
-// Skinny products (a decode step: M <= a few hundred rows against a large weight) have too few
-// output tiles to occupy 148 SMs, and each CTA would stream its whole K extent at one SM's share
-// of the HBM bandwidth. Split-K gives every (tile, K-slice) pair its own CTA: slice s of tile
-// (m, n) is the virtual row block s * tiles_m + m, its partial sums go to an fp32 workspace
-// [S, tiles_m * 128, N] and a small kernel adds the slices (+ bias) into the bf16 output.
+// Skinny products (a decode step: M <= a few hundred rows against a large weight) are a read of the weight. Its rows are
+// the 128-row side of the tile, the M rows the narrow one (BN = 32 .. 128), so that little of the tensor cores' and none of
+// the workspace's work is padding, and a lane of the epilogue owns a column of the output: the partial sums leave in
+// coalesced rows. There are too few such tiles to occupy 148 SMs, and each CTA would stream its whole K extent at one
+// SM's share of the HBM bandwidth, so K is split as well: slice s of weight rows n is the virtual row block s * tiles_n + n, its partial
+// sums go to an fp32 workspace [S, M, N], and a small kernel adds the slices (+ bias) into the bf16 output. With the
+// M rows on the 128-row side, as this was before, one row wrote 127 rows of padding beside it: the four projections of a
+// Qwen3-1.7B layer took 48 us for one row, now 31 us, and launched as dependents of one another (the weight is on its way
+// while the small kernels before still run) a decode step takes 1.52 ms instead of 1.82 ms.
 struct SplitKEpi {
-  StoreEpi st;   // writes the fp32 workspace, M = S * tiles_m * 128
-  int tiles_m_real, kper, kblocks_total;
-  using State = StoreEpi::State;
+  float* ws;
+  int M, N;       // rows of the input and of the weight
+  int tiles_n, kper, kblocks_total;
+  static constexpr bool kChained = true;
+  struct State {};
 
-  __device__ __forceinline__ bool tile(int cta, int ncta, int it, int tiles_m_virtual, int tiles_n, int& m_blk,
-                                       int& n_blk) const {
+  __device__ __forceinline__ bool tile(int cta, int ncta, int it, int tiles_virtual, int tiles_m, int& n_blk,
+                                       int& m_blk) const {
     const long long t = static_cast<long long>(it) * ncta + cta;
-    if (t >= static_cast<long long>(tiles_m_virtual) * tiles_n) return false;
-    // consecutive CTAs take the K slices of one output tile, then the next column block
-    m_blk = static_cast<int>(t % tiles_m_virtual);
-    n_blk = static_cast<int>(t / tiles_m_virtual);
+    if (t >= static_cast<long long>(tiles_virtual) * tiles_m) return false;
+    // CTAs that run together read the weight in one sweep; its rows come past again for the next block of the input
+    n_blk = static_cast<int>(t % tiles_virtual);
+    m_blk = static_cast<int>(t / tiles_virtual);
     return true;
   }
-  __device__ __forceinline__ int a_m0(int mv) const { return (mv % tiles_m_real) * kBM; }
-  __device__ __forceinline__ int k_begin(int mv) const { return (mv / tiles_m_real) * kper * kBK; }
-  __device__ __forceinline__ int k_blocks(int mv) const {
-    const int left = kblocks_total - (mv / tiles_m_real) * kper;
+  __device__ __forceinline__ int a_m0(int nv) const { return (nv % tiles_n) * kBM; }
+  __device__ __forceinline__ int k_begin(int nv) const { return (nv / tiles_n) * kper * kBK; }
+  __device__ __forceinline__ int k_blocks(int nv) const {
+    const int left = kblocks_total - (nv / tiles_n) * kper;
     return left < kper ? (left > 0 ? left : 0) : kper;
   }
   __device__ __forceinline__ bool gate(int, int, volatile int*, int*) const { return true; }
   __device__ __forceinline__ void begin(State&, int, int, int) const {}
   __device__ __forceinline__ void end(State&, int, int, int) const {}
-  __device__ __forceinline__ void chunk(State& s, int row, int col0, const float (&v)[32]) const {
-    st.chunk(s, row, col0, v);
+  __device__ __forceinline__ void chunk(State&, int row, int col0, const float (&v)[32]) const {
+    const int nv = row / kBM, n = row - (nv - nv % tiles_n) * kBM;
+    if (n >= N) return;
+    float* out = ws + (static_cast<long long>(nv / tiles_n) * M + col0) * N + n;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (col0 + i < M) out[static_cast<long long>(i) * N] = v[i];
   }
 };
 
@@ -350,10 +379,13 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, const __nv_bf
                                      long long slice_stride) {
   const int nq = N >> 2;
   const long long total = static_cast<long long>(M) * nq;
+  pdl_wait();
+  pdl_trigger();
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int row = static_cast<int>(i / nq), c = static_cast<int>(i % nq) * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (int s = 0; s < S; ++s) {
       const float4 v = *reinterpret_cast<const float4*>(ws + s * slice_stride + static_cast<long long>(row) * N + c);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
@@ -390,6 +422,38 @@ __global__ void splitk_reduce_glu_kernel(const float* __restrict__ ws, __nv_bflo
   }
 }
 
+// Split-K reduction of a fused gate / up projection (gate: the first I columns, up: the last) with SwiGLU behind it. The two
+// halves are rounded to bf16 first, as the projection's output is, so the result is that of the separate kernels.
+__global__ void __launch_bounds__(256)
+splitk_reduce_swiglu_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int M, int I, int S,
+                            long long slice_stride) {
+  const int nq = I >> 2;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
+  pdl_wait();
+  pdl_trigger();
+  if (i >= nq) return;
+  const float* g = ws + static_cast<long long>(row) * 2 * I + 4 * i;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 4
+  for (int s = 0; s < S; ++s) {
+    const float4 x = *reinterpret_cast<const float4*>(g + s * slice_stride);
+    const float4 y = *reinterpret_cast<const float4*>(g + s * slice_stride + I);
+    a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+    b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+  }
+  auto act = [](float gate, float up) {
+    gate = __bfloat162float(__float2bfloat16(gate));
+    up = __bfloat162float(__float2bfloat16(up));
+    return gate * sigmoid_rcp(gate) * up;
+  };
+  __nv_bfloat162 lo = __floats2bfloat162_rn(act(a.x, b.x), act(a.y, b.y));
+  __nv_bfloat162 hi = __floats2bfloat162_rn(act(a.z, b.z), act(a.w, b.w));
+  uint2 pk;
+  pk.x = *reinterpret_cast<uint32_t*>(&lo);
+  pk.y = *reinterpret_cast<uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(out + static_cast<long long>(row) * I + 4 * i) = pk;
+}
+
 // Split-K reduction fused with the residual add and RMSNorm that follow a projection in a decoder
 // block: a group of threads per row (common/rms_row.cuh) sums the S fp32 slices (+ bias), rounds to bf16 (the
 // projection's output precision), adds the bf16 residual stream, stores the new residual (bf16) and the normalised row.
@@ -406,10 +470,12 @@ splitk_reduce_rmsnorm_kernel(const float* __restrict__ ws, const __nv_bfloat16* 
   __shared__ float part[8][kRmsMaxWarps];
   const int tid = threadIdx.x, group = blockDim.x;
   const long long row = static_cast<long long>(blockIdx.x) * blockDim.y + threadIdx.y;
-  if (row >= M) return;  // the whole group
   const int nvec = N >> 3;
   float v[VPT][8], ss = 0.f;
   uint4 wraw[VPT];
+  pdl_wait();
+  pdl_trigger();
+  if (row >= M) return;  // the whole group
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = tid + group * i;
@@ -615,6 +681,11 @@ int b200_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int 
   if (bn == 128) {
     DISPATCH(128)
   }
+  if (bn == 512) {  // 256 x 256 on a pair of SMs
+    auto go = a_mn ? (b_mn ? launch_pair<true, true> : launch_pair<true, false>)
+                   : (b_mn ? launch_pair<false, true> : launch_pair<false, false>);
+    return go(A, B, C, bias, M, N, K, lda, ldb, ldc, out_fp32, accumulate, stream);
+  }
   DISPATCH(256)
 #undef DISPATCH
 }
@@ -704,59 +775,73 @@ int b200_gemm_grouped_wgrad(const void* dY, const void* X, void* dW, const int* 
   return 0;
 }
 
-// Launches the split-K GEMM proper: fp32 partial tiles into `workspace`. Returns the number of slices
+}  // extern "C"
+
+// Launches the split-K GEMM proper: fp32 partial sums into `workspace` [S, M, N]. Returns the number of slices
 // through *S_out and the slice stride (elements) through *stride_out.
-static int launch_splitk_partials(const void* A, const void* B, float* workspace, int M, int N, int K, long long lda,
-                                  long long ldb, int splits, int* S_out, long long* stride_out, cudaStream_t stream) {
+template <int BN>
+static int launch_splitk_bn(const void* A, const void* B, float* workspace, int M, int N, int K, long long lda,
+                            long long ldb, int kper, int S, bool chained, cudaStream_t stream) {
   using namespace b200;
-  constexpr int BN = 128;
   using Cfg = GemmCfg<BN>;
-  const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + BN - 1) / BN;
-  const int kblocks = (K + kBK - 1) / kBK;
-  const int kper = (kblocks + splits - 1) / splits;
-  const int S = (kblocks + kper - 1) / kper;  // slices that actually hold work
-  const int Mv = S * tiles_m * kBM;
-  CUtensorMap tmA, tmB;
-  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda * 2, kBM, 64);
+  const int tiles_n = (N + kBM - 1) / kBM, tiles_m = (M + BN - 1) / BN;
+  CUtensorMap tmW, tmX;
+  int rc = make_tmap_2d(&tmW, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb * 2, kBM, 64);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb * 2, BN, 64);
+  rc = make_tmap_2d(&tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda * 2, BN, 64);
   if (rc) return rc;
-  SplitKEpi epi{StoreEpi{workspace, nullptr, N, Mv, N, 1, 0}, tiles_m, kper, kblocks};
+  const SplitKEpi epi{workspace, M, N, tiles_n, kper, (K + kBK - 1) / kBK};
   auto kern = gemm_tcgen05_kernel<BN, false, false, SplitKEpi>;
   static bool attr_set = false;
   if (!attr_set) {
     B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set = true;
   }
-  const long long tiles = static_cast<long long>(S) * tiles_m * tiles_n;
+  const long long tiles = static_cast<long long>(S) * tiles_n * tiles_m;
   const int grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
   int* status = device_status_word();
   if (!status) return -3;
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(tmA, tmB, Mv, N, K, epi, status);
-  B200_CHECK(cudaGetLastError());
-  *S_out = S;
-  *stride_out = static_cast<long long>(tiles_m) * kBM * N;
+  B200_CHECK(launch_kernel(kern, grid, kGemmThreads, Cfg::kSmemBytes, stream, chained, tmW, tmX, S * tiles_n * kBM, M, K, epi,
+                           status));
   return 0;
 }
 
+static int launch_splitk_partials(const void* A, const void* B, float* workspace, int M, int N, int K, long long lda,
+                                  long long ldb, int splits, int* S_out, long long* stride_out, cudaStream_t stream,
+                                  bool chained = false) {
+  using namespace b200;
+  const int kblocks = (K + kBK - 1) / kBK;
+  const int kper = (kblocks + splits - 1) / splits;
+  const int S = (kblocks + kper - 1) / kper;  // slices that actually hold work
+  *S_out = S;
+  *stride_out = static_cast<long long>(M) * N;
+  if (M <= 32) return launch_splitk_bn<32>(A, B, workspace, M, N, K, lda, ldb, kper, S, chained, stream);
+  if (M <= 64) return launch_splitk_bn<64>(A, B, workspace, M, N, K, lda, ldb, kper, S, chained, stream);
+  // (256-wide tiles for more rows: a CTA's only tile then ends in 128 KB of partial sums that nothing overlaps)
+  return launch_splitk_bn<128>(A, B, workspace, M, N, K, lda, ldb, kper, S, chained, stream);
+}
+
+extern "C" {
+
+// chained (here and below): launch as programmatic dependents; the kernel before them in the stream must not write B.
 // C[M,N] (bf16) = A[M,K] . B[N,K]^T (+ bias) with the K extent split over `splits` CTAs per tile.
-// workspace: fp32 [splits * ceil(M/128)*128 * N]. N % 4 == 0, ldc % 4 == 0.
+// workspace: fp32 [splits * M * N]. N % 4 == 0, ldc % 4 == 0.
 int b200_gemm_bf16_splitk(const void* A, const void* B, void* C, const void* bias, float* workspace, int M, int N,
-                          int K, long long lda, long long ldb, long long ldc, int splits, cudaStream_t stream) {
+                          int K, long long lda, long long ldb, long long ldc, int splits, int chained,
+                          cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (N & 3) || (ldc & 3) || splits < 1) return -100;
   int S = 0;
   long long stride = 0;
-  const int rc = launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, &S, &stride, stream);
+  const int rc = launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, &S, &stride, stream, chained);
   if (rc) return rc;
   const long long total = static_cast<long long>(M) * (N >> 2);
   long long rg = (total + 255) / 256;
   const long long maxg = static_cast<long long>(sm_count()) * 8;
   if (rg > maxg) rg = maxg;
-  splitk_reduce_kernel<false><<<(unsigned)rg, 256, 0, stream>>>(workspace, (const __nv_bfloat16*)bias, (__nv_bfloat16*)C, ldc,
-                                                        M, N, S, stride);
-  B200_CHECK(cudaGetLastError());
+  B200_CHECK(launch_kernel(splitk_reduce_kernel<false>, (unsigned)rg, 256, 0, stream, chained, workspace,
+                           (const __nv_bfloat16*)bias, (__nv_bfloat16*)C, ldc, M, N, S, stride));
   return 0;
 }
 
@@ -768,30 +853,46 @@ int b200_gemm_bf16_splitk_partials(const void* A, const void* B, float* workspac
   return launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, S_out, stride_out, stream);
 }
 
+// out [M, I] (bf16) = silu(gate) * up of the fused projection A . B^T, B [2 * I, K], with the activation in the split-K
+// reduction. I % 4 == 0; workspace as above with N = 2 * I; M <= 65535.
+int b200_gemm_bf16_splitk_swiglu(const void* A, const void* B, void* out, float* workspace, int M, int I, int K,
+                                 long long lda, long long ldb, int splits, int chained,
+                                 cudaStream_t stream) {
+  using namespace b200;
+  if (M <= 0 || I <= 0 || K <= 0) return 0;
+  if ((lda & 7) || (ldb & 7) || (I & 3) || splits < 1 || M > 65535) return -100;
+  int S = 0;
+  long long stride = 0;
+  const int rc = launch_splitk_partials(A, B, workspace, M, 2 * I, K, lda, ldb, splits, &S, &stride, stream, chained);
+  if (rc) return rc;
+  B200_CHECK(launch_kernel(splitk_reduce_swiglu_kernel, dim3((I / 4 + 255) / 256, M), 256, 0, stream, chained, workspace,
+                           (__nv_bfloat16*)out, M, I, S, stride));
+  return 0;
+}
+
 // Split-K projection followed, in the reduction kernel, by the residual add and RMSNorm:
 //   h = bf16(A . B^T + bias) + residual;  res_out = bf16(h);  y = rmsnorm(res_out) * norm_w
 // residual may be null (then res_out = bf16(A . B^T + bias)). y and res_out are contiguous [M, N] bf16;
 // N % 8 == 0 and N <= 8192. Two launches instead of three (GEMM, reduce, norm).
 int b200_gemm_bf16_splitk_rmsnorm(const void* A, const void* B, const void* bias, float* workspace, int M, int N, int K,
                                   long long lda, long long ldb, int splits, const void* residual, const void* norm_w,
-                                  void* y, void* res_out, float eps, cudaStream_t stream) {
+                                  void* y, void* res_out, float eps, int chained, cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (N & 7) || N > 8192 || splits < 1) return -100;
   int S = 0;
   long long stride = 0;
-  const int rc = launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, &S, &stride, stream);
+  const int rc = launch_splitk_partials(A, B, workspace, M, N, K, lda, ldb, splits, &S, &stride, stream, chained);
   if (rc) return rc;
   const RmsShape shape = rms_shape(N);
   const int rows = 256 / shape.group > 1 ? 256 / shape.group : 1;
 #define B200_LAUNCH_RN(VPT_)                                                                                 \
-  splitk_reduce_rmsnorm_kernel<VPT_><<<(M + rows - 1) / rows, dim3(shape.group, rows), 0, stream>>>(         \
+  B200_CHECK(launch_kernel(splitk_reduce_rmsnorm_kernel<VPT_>, (M + rows - 1) / rows, dim3(shape.group, rows), 0, stream, chained, \
       workspace, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)norm_w,   \
-      (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, M, N, S, stride, eps)
+      (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, M, N, S, stride, eps))
   if (shape.vpt == 1) B200_LAUNCH_RN(1);
   else B200_LAUNCH_RN(2);
 #undef B200_LAUNCH_RN
-  B200_CHECK(cudaGetLastError());
   return 0;
 }
 
@@ -825,7 +926,7 @@ static int launch_epi(const void* A, const void* B, const Epi& epi, int M, int N
 extern "C" {
 
 // A [M, K] . B [N, K]^T with the DytEpi tail: res [M, N] fp32 (in place), y [M, N] bf16, N % 4 == 0. splits > 1: split-K
-// into `workspace` (fp32 [splits * ceil(M/128)*128 * N]) with the tail in the reduction kernel.
+// into `workspace` (fp32 [splits * M * N]) with the tail in the reduction kernel.
 int b200_gemm_bf16_dyt(const void* A, const void* B, float* workspace, int M, int N, int K, long long lda,
                        long long ldb, int splits, const void* scale, float* res, const void* alpha, const void* w,
                        const void* b, void* y, cudaStream_t stream) {

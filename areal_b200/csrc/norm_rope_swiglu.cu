@@ -16,7 +16,9 @@
 #include <stdint.h>
 
 #include "common/host_utils.h"
+#include "common/ptx.cuh"
 #include "common/rms_row.cuh"
+#include "common/sigmoid.cuh"
 
 namespace b200 {
 
@@ -362,6 +364,8 @@ qknorm_rope_kvwrite_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfl
   const int t = static_cast<int>(gw / groups);
   const int h = static_cast<int>(gw % groups) * kRopeHeads + (lane >> 3);
   const int hs = min(h, heads - 1);
+  pdl_wait();
+  pdl_trigger();
   const long long slot = slot_mapping[t];
   const __nv_bfloat16* src = qkv + (static_cast<long long>(t) * heads + hs) * D;
   const BF8 raw_a = reinterpret_cast<const BF8*>(src)[l], raw_b = reinterpret_cast<const BF8*>(src + 64)[l];
@@ -495,12 +499,6 @@ qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16
 // sigmoid is one approximate reciprocal (1 ulp; the exponential before it is no better), because IEEE divisions alone kept
 // the issue slots busy for most of the time that the memory needs. Two rows a thread; one is 4% slower, four 30%. 16384 x 6144:
 // 129 us forward and 181 us backward before, 96 and 146 us (6.3 and 6.9 TB/s) now.
-__device__ __forceinline__ float sigmoid_rcp(float x) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-x)));
-  return r;
-}
-
 template <int ROWS>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I) {
@@ -650,18 +648,17 @@ int b200_qknorm_rope_fwd(const void* qkv, const void* qw, const void* kw, const 
 int b200_qknorm_rope_kvwrite(const void* qkv, const void* qw, const void* kw, const float* cos_t,
                              const float* sin_t, const int* pos, void* q_out, const long long* slot_mapping,
                              void* k_cache, void* v_cache, int T, int Hq, int Hkv, int D, int block_size,
-                             float eps, int has_norm, cudaStream_t stream) {
+                             float eps, int has_norm, int chained, cudaStream_t stream) {
   using namespace b200;
   if (D != 128) return -100;
   if (T == 0) return 0;
   const long long warps = static_cast<long long>(T) * ((Hq + 2 * Hkv + kRopeHeads - 1) / kRopeHeads);
   const int tpb = 128;
   const long long grid = (warps * 32 + tpb - 1) / tpb;
-  qknorm_rope_kvwrite_kernel<<<(unsigned)grid, tpb, 0, stream>>>(
-      (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cos_t, sin_t, pos,
-      (__nv_bfloat16*)q_out, slot_mapping, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, T, Hq, Hkv,
-      block_size, eps, has_norm);
-  B200_CHECK(cudaGetLastError());
+  B200_CHECK(launch_kernel(qknorm_rope_kvwrite_kernel, (unsigned)grid, tpb, 0, stream, chained, (const __nv_bfloat16*)qkv,
+                           (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, cos_t, sin_t, pos, (__nv_bfloat16*)q_out,
+                           slot_mapping, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, T, Hq, Hkv, block_size, eps,
+                           has_norm));
   return 0;
 }
 

@@ -97,14 +97,6 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
   const int b = blockIdx.x, hk = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = seq_lens[b];
-  const int slabs_total = (L + kSlab - 1) / kSlab;
-  const int per = (slabs_total + nsplit - 1) / nsplit;
-  const int s_begin = split * per;
-  const int s_end = min(slabs_total, s_begin + per);
-  const int spp = block_size / kSlab;  // slabs per page
-  const int* bt = block_table + static_cast<long long>(b) * max_blocks;
-
   if (threadIdx.x == 0) {
     for (int i = 0; i < kWarpsD * kSlots; ++i) mbar_init(&bars[i], 1);
     *abort_flag = 0;
@@ -112,6 +104,15 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
   }
+  pdl_wait();
+  pdl_trigger();
+  const int L = seq_lens[b];
+  const int slabs_total = (L + kSlab - 1) / kSlab;
+  const int per = (slabs_total + nsplit - 1) / nsplit;
+  const int s_begin = split * per;
+  const int s_end = min(slabs_total, s_begin + per);
+  const int spp = block_size / kSlab;  // slabs per page
+  const int* bt = block_table + static_cast<long long>(b) * max_blocks;
   __syncthreads();
 
   uint8_t* ring = dsm + warp * kSlots * kSlabB;
@@ -271,6 +272,8 @@ __global__ void paged_decode_merge_kernel(const float* __restrict__ o_part,
                                           __nv_bfloat16* __restrict__ out, int nsplit) {
   const long long bh = blockIdx.x;  // (b * Hq + h)
   const int d = threadIdx.x;        // 128 threads
+  pdl_wait();
+  pdl_trigger();
   float mn = -INFINITY;
   for (int s = 0; s < nsplit; ++s) mn = fmaxf(mn, ml_part[(bh * nsplit + s) * 2]);
   float lt = 0.f, at = 0.f;
@@ -305,11 +308,12 @@ int b200_kv_cache_write(const void* k, const void* v, long long ldk, long long l
 }
 
 // k_cache / v_cache: [num_blocks, Hkv, block_size, 128] bf16, block_size a multiple of 16.
-// o_part: fp32 [B, Hq, nsplit, 128]; ml_part: fp32 [B, Hq, nsplit, 2] (unused when nsplit == 1).
+// o_part: fp32 [B, Hq, nsplit, 128]; ml_part: fp32 [B, Hq, nsplit, 2] (unused when nsplit == 1). chained: launch as
+// programmatic dependents.
 int b200_paged_decode(const void* q, const void* k_cache, const void* v_cache,
                       const int* block_table, const int* seq_lens, void* out, float* o_part,
                       float* ml_part, int B, int Hq, int Hkv, int D, int block_size, int num_blocks,
-                      int max_blocks, int nsplit, float softmax_scale, cudaStream_t stream) {
+                      int max_blocks, int nsplit, float softmax_scale, int chained, cudaStream_t stream) {
   using namespace b200;
   if (D != kHD || Hq % Hkv || block_size % kSlab) return -100;
   if (B == 0) return 0;
@@ -326,9 +330,9 @@ int b200_paged_decode(const void* q, const void* k_cache, const void* v_cache,
   dim3 grid(B, Hkv, nsplit);
 #define LAUNCH(G_)                                                                                        \
   cudaFuncSetAttribute(paged_decode_kernel<G_>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecodeSmem); \
-  paged_decode_kernel<G_><<<grid, kWarpsD * 32, kDecodeSmem, stream>>>(                                   \
+  B200_CHECK(launch_kernel(paged_decode_kernel<G_>, grid, kWarpsD * 32, kDecodeSmem, stream, chained,     \
       tmK, tmV, (const __nv_bfloat16*)q, block_table, seq_lens, (__nv_bfloat16*)out, o_part, ml_part, Hq, \
-      Hkv, block_size, max_blocks, nsplit, sl2, status)
+      Hkv, block_size, max_blocks, nsplit, sl2, status))
   switch (G) {
     case 1: LAUNCH(1); break;
     case 2: LAUNCH(2); break;
@@ -338,11 +342,9 @@ int b200_paged_decode(const void* q, const void* k_cache, const void* v_cache,
     default: return -101;
   }
 #undef LAUNCH
-  B200_CHECK(cudaGetLastError());
-  if (nsplit > 1) {
-    paged_decode_merge_kernel<<<B * Hq, kHD, 0, stream>>>(o_part, ml_part, (__nv_bfloat16*)out, nsplit);
-    B200_CHECK(cudaGetLastError());
-  }
+  if (nsplit > 1)
+    B200_CHECK(launch_kernel(paged_decode_merge_kernel, B * Hq, kHD, 0, stream, chained, o_part, ml_part, (__nv_bfloat16*)out,
+                             nsplit));
   return 0;
 }
 

@@ -26,7 +26,7 @@ import torch.nn.functional as F
 
 from ..ops import _lib, fused
 from ..ops.attention import VarlenMeta, varlen_attention
-from ..ops.gemm import gemm, linear, linear_rmsnorm
+from ..ops.gemm import gemm, linear, linear_rmsnorm, linear_swiglu
 from ..ops.rollout_ops import kv_cache_write, paged_decode
 from .config import ModelConfig
 
@@ -93,11 +93,15 @@ class Attention(nn.Module):
             q, k, v = self.project_qkv(x, cos, sin, pos)
             kv_cache_write(k, v, slot_mapping, k_cache, v_cache)
             return q
-        qkv = _dense(x, self.qkv, self.qkv_bias, cfg)
+        # a decode step's kernels are launched as programmatic dependents of one another (none of them writes a weight)
+        if x.is_cuda and x.dtype == torch.bfloat16 and not cfg.fp8:
+            qkv = gemm(x, self.qkv, bias=self.qkv_bias, chained=True)
+        else:
+            qkv = _dense(x, self.qkv, self.qkv_bias, cfg)
         if self.lora_qkv is not None:
             qkv = qkv + self.lora_qkv(x)
         return fused.qknorm_rope_kvwrite(qkv, self.q_norm, self.k_norm, cos, sin, pos, self.n_q, self.n_kv,
-                                         cfg.head_dim, cfg.rms_norm_eps, slot_mapping, k_cache, v_cache)
+                                         cfg.head_dim, cfg.rms_norm_eps, slot_mapping, k_cache, v_cache, chained=True)
 
     def _fused_ulysses(self, x, cos, sin, pos, meta, attn_fn=None):
         """Ulysses with the projection and the sequence→head exchange fused into one kernel: the
@@ -680,11 +684,12 @@ class QwenModel(nn.Module):
                 continue
             q = layer.attn.project_q_write_kv(y, cos, sin, pos, slot_mapping, kv_caches[i][0], kv_caches[i][1])
             a = paged_decode(q, kv_caches[i][0], kv_caches[i][1], block_table, seq_lens,
-                             max_seq_len=max_seq_len)
+                             max_seq_len=max_seq_len, chained=plain)
             if hasattr(layer.attn, "out_proj"):  # latent attention: drops the value padding itself
                 y, res = fused.rmsnorm(layer.attn.out_proj(a), layer.post_norm, layer.eps, residual=res)
             elif plain and layer.attn.lora_o is None:
-                y, res = linear_rmsnorm(a.reshape(a.shape[0], -1), layer.attn.o, layer.post_norm, layer.eps, res)
+                y, res = linear_rmsnorm(a.reshape(a.shape[0], -1), layer.attn.o, layer.post_norm, layer.eps, res,
+                                        chained=True)
             else:
                 y, res = fused.rmsnorm(linear(a.reshape(a.shape[0], -1), layer.attn.o), layer.post_norm, layer.eps,
                                        residual=res)
@@ -692,8 +697,8 @@ class QwenModel(nn.Module):
             if plain and isinstance(m, DenseMLP) and m.lora_gate_up is None and m.lora_down is None:
                 nxt_w, nxt_eps = ((self.layers[i + 1].input_norm, self.layers[i + 1].eps) if i + 1 < n_layers
                                   else (self.norm, self.cfg.rms_norm_eps))
-                h = fused.swiglu(linear(y, m.gate_up))
-                y, res = linear_rmsnorm(h, m.down, nxt_w, nxt_eps, res)
+                h = linear_swiglu(y, m.gate_up, chained=True)
+                y, res = linear_rmsnorm(h, m.down, nxt_w, nxt_eps, res, chained=True)
                 x = None
             else:
                 x = m(y)

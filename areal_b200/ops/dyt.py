@@ -78,7 +78,7 @@ def linear_residual_dyt(a: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, r
             and w.data_ptr() % 16 == 0):
         return residual_dyt(linear(a, w), scale, res, norm)
     splits = _splitk_plan(M, N, K)
-    ws = torch.empty((splits * -(-M // 128) * 128, N), dtype=torch.float32, device=a.device) if splits else None
+    ws = torch.empty((splits * M, N), dtype=torch.float32, device=a.device) if splits else None
     y = torch.empty((M, N), dtype=a.dtype, device=a.device)
     rc = _lib.kernels().b200_gemm_bf16_dyt(
         _lib.ptr(a), _lib.ptr(w), _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),

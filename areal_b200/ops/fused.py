@@ -246,10 +246,11 @@ def qknorm_rope(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps=1e-6):
 
 
 @torch.no_grad()
-def qknorm_rope_kvwrite(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps, slot_mapping, k_cache, v_cache):
+def qknorm_rope_kvwrite(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps, slot_mapping, k_cache, v_cache, chained=False):
     """Inference form of :func:`qknorm_rope`: returns ``q [T, Hq, D]`` and writes the normalised,
     rotated ``k`` and the raw ``v`` into the paged caches ``[num_blocks, Hkv, block_size, D]`` at
-    ``slot_mapping [T]`` (int64, negative = skip) in the same kernel."""
+    ``slot_mapping [T]`` (int64, negative = skip) in the same kernel. ``chained``: launched as a programmatic dependent of
+    the kernel before it."""
     if not (_lib.use_cuda_kernels(qkv, k_cache) and qkv.dtype == torch.bfloat16 and D == 128 and qkv.is_contiguous()
             and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0):
         from .rollout_ops import kv_cache_write
@@ -271,7 +272,7 @@ def qknorm_rope_kvwrite(qkv, qw, kw, cos, sin, pos, Hq, Hkv, D, eps, slot_mappin
         _lib.ptr(qkv), _lib.ptr(qw), _lib.ptr(kw), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(pos), _lib.ptr(q),
         _lib.ptr(slots.contiguous()), _lib.ptr(k_cache), _lib.ptr(v_cache), ctypes.c_int(T), ctypes.c_int(Hq),
         ctypes.c_int(Hkv), ctypes.c_int(D), ctypes.c_int(k_cache.shape[2]), ctypes.c_float(eps),
-        ctypes.c_int(int(qw is not None)), _lib.stream_ptr())
+        ctypes.c_int(int(qw is not None)), ctypes.c_int(int(chained)), _lib.stream_ptr())
     _lib.check(rc, "b200_qknorm_rope_kvwrite")
     _lib.count_launch()
     return q

@@ -16,6 +16,7 @@ Counterpart of the cuBLAS-backed ``nn.Linear`` calls of the reference
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 
 import torch
@@ -49,12 +50,14 @@ def gemm(
     out_dtype: torch.dtype = torch.bfloat16,
     accumulate: bool = False,
     bn: int = 0,
+    chained: bool = False,
 ) -> torch.Tensor:
     """``C[M,N] = A B^T (+bias)``.
 
     ``a`` is ``[M,K]`` (``a_mn=False``) or ``[K,M]`` (``a_mn=True``); ``b`` is ``[N,K]``
     or ``[K,N]`` likewise. ``out`` may be a bf16 or fp32 2-D tensor with unit
-    inner stride; ``accumulate`` adds to it.
+    inner stride; ``accumulate`` adds to it. ``chained`` (skinny products): launched as programmatic dependents of the
+    kernel before, which must not write ``b``; the weight is on its way while that kernel still runs.
     """
     if not _lib.use_cuda_kernels(a, b):
         return _gemm_ref(a, b, a_mn, b_mn, bias, out_dtype, out, accumulate)
@@ -88,16 +91,15 @@ def gemm(
         if not a_mn:
             K = a.shape[1]
     # skinny products (decode steps): too few output tiles for 148 SMs ⇒ split the K extent
-    if (bn == 0 and not a_mn and not b_mn and not accumulate and out.dtype == torch.bfloat16 and M <= 512
-            and N % 4 == 0 and out.stride(0) % 4 == 0 and not need_pad and K >= 1024):
-        tiles = -(-M // 128) * -(-N // 128)
-        splits = min(8, 148 // tiles, K // 256)
-        if splits >= 2:
-            ws = torch.empty((splits * -(-M // 128) * 128, N), dtype=torch.float32, device=a.device)
+    if (bn == 0 and not a_mn and not b_mn and not accumulate and out.dtype == torch.bfloat16 and out.stride(0) % 4 == 0
+            and not need_pad):
+        splits = _splitk_plan(M, N, K)
+        if splits:
+            ws = torch.empty((splits * M, N), dtype=torch.float32, device=a.device)
             rc = _lib.kernels().b200_gemm_bf16_splitk(
                 _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias), _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N),
                 ctypes.c_int(K), ctypes.c_longlong(a.stride(0)), ctypes.c_longlong(b.stride(0)),
-                ctypes.c_longlong(out.stride(0)), ctypes.c_int(splits), _lib.stream_ptr())
+                ctypes.c_longlong(out.stride(0)), ctypes.c_int(splits), ctypes.c_int(int(chained)), _lib.stream_ptr())
             _lib.check(rc, "b200_gemm_bf16_splitk")
             _lib.count_launch(2)
             return out
@@ -125,12 +127,23 @@ def gemm(
     return out
 
 
+@functools.lru_cache(maxsize=4096)
 def _splitk_plan(M: int, N: int, K: int) -> int:
-    """Number of K splits the skinny-GEMM path uses for this shape (0: not a split-K shape)."""
+    """Number of K slices of the skinny path for this shape (0: not a shape for it). The kernel walks items of 128 weight
+    rows by a K slice, one CTA per SM, so a pass takes ``rounds of items * (reduction blocks of an item + its start)``; what is saved
+    there by more slices is paid for with partial sums that are written and read back. Up to 128 rows the two are weighed in bytes
+    (the sums at half price: they stay in L2). With more rows the sums of many slices cost more than they save (a decode step of
+    256 rows of Qwen3-1.7B: 8.45 ms by that rule, 7.49 ms with slices for a single round of items), and a product with as
+    many tiles as half the SMs is not split."""
     if M > 512 or N % 4 or K < 1024:
         return 0
-    tiles = -(-M // 128) * -(-N // 128)
-    splits = min(8, 148 // tiles, K // 256)
+    tiles, blocks = -(-M // 128) * -(-N // 128), -(-K // 64)
+    if M > 128:
+        splits = min(8, 148 // tiles, K // 256)
+    else:
+        rows = 32 if M <= 32 else 64 if M <= 64 else 128
+        splits = min(range(1, min(16, blocks // 2) + 1),
+                     key=lambda s: -(-tiles * s // 148) * (-(-blocks // s) + 2) * 148 * (128 + rows / 2) * 128 + 4 * s * M * N)
     return splits if splits >= 2 else 0
 
 
@@ -165,7 +178,7 @@ def linear_slices(x: torch.Tensor, w: torch.Tensor) -> "torch.Tensor | Slices":
     splits = _splitk_plan(M, N, K) if x.dtype == torch.bfloat16 and _lib.use_cuda_kernels(x, w) else 0
     if not (splits and K % 8 == 0 and _tma_rows(x, w)):
         return linear(x, w)
-    ws = torch.empty((splits * -(-M // 128) * 128, N), dtype=torch.float32, device=x.device)
+    ws = torch.empty((splits * M, N), dtype=torch.float32, device=x.device)
     S, stride = ctypes.c_int(0), ctypes.c_longlong(0)
     rc = _lib.kernels().b200_gemm_bf16_splitk_partials(
         _lib.ptr(x), _lib.ptr(w), _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
@@ -193,7 +206,7 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         _lib.count_launch()
         return z
     splits = _splitk_plan(M, N, K)
-    ws = torch.empty((splits * -(-M // 128) * 128, N), dtype=torch.float32, device=x.device) if splits else None
+    ws = torch.empty((splits * M, N), dtype=torch.float32, device=x.device) if splits else None
     y = torch.empty((M, N), dtype=x.dtype, device=x.device)
     rc = _lib.kernels().b200_gemm_bf16_relu2(
         _lib.ptr(x), _lib.ptr(w), _lib.ptr(y), _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
@@ -205,11 +218,11 @@ def linear_relu2(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 @torch.no_grad()
 def linear_rmsnorm(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor, eps: float,
-                   residual: torch.Tensor | None = None):
+                   residual: torch.Tensor | None = None, chained: bool = False):
     """``h = x @ w.T (+ residual)``; returns ``(rmsnorm(h) * norm_w, h)``: a decoder block's projection,
     residual add and following norm. For skinny (decode-step) shapes the residual add and the norm
     run inside the split-K reduction kernel (two launches instead of three, bit-identical results);
-    other shapes run the separate kernels. Inference only."""
+    other shapes run the separate kernels. Inference only. ``chained`` as in :func:`gemm`."""
     from . import fused
 
     M, K = x.shape
@@ -223,16 +236,38 @@ def linear_rmsnorm(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor, eps: 
         if residual is None:
             return fused.rmsnorm(a, norm_w, eps), a
         return fused.rmsnorm(a, norm_w, eps, residual=residual)
-    ws = torch.empty((splits * -(-M // 128) * 128, N), dtype=torch.float32, device=x.device)
+    ws = torch.empty((splits * M, N), dtype=torch.float32, device=x.device)
     y = torch.empty((M, N), dtype=x.dtype, device=x.device)
     res_out = torch.empty((M, N), dtype=x.dtype, device=x.device)
     rc = _lib.kernels().b200_gemm_bf16_splitk_rmsnorm(
         _lib.ptr(x), _lib.ptr(w), None, _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
         ctypes.c_longlong(x.stride(0)), ctypes.c_longlong(w.stride(0)), ctypes.c_int(splits), _lib.ptr(residual),
-        _lib.ptr(norm_w), _lib.ptr(y), _lib.ptr(res_out), ctypes.c_float(eps), _lib.stream_ptr())
+        _lib.ptr(norm_w), _lib.ptr(y), _lib.ptr(res_out), ctypes.c_float(eps), ctypes.c_int(int(chained)), _lib.stream_ptr())
     _lib.check(rc, "b200_gemm_bf16_splitk_rmsnorm")
     _lib.count_launch(2)
     return y, res_out
+
+
+@torch.no_grad()
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor, chained: bool = False) -> torch.Tensor:
+    """``swiglu(x @ w.T)`` of a fused gate / up projection; for decode-sized products SwiGLU runs in the split-K reduction
+    (the halves are rounded to bf16 in between, as by the separate kernels). Inference only. ``chained`` as in :func:`gemm`."""
+    from . import fused
+
+    M, K = x.shape
+    N = w.shape[0]
+    splits = _splitk_plan(M, N, K) if x.dtype == torch.bfloat16 and _lib.use_cuda_kernels(x, w) else 0
+    if not (splits and N % 16 == 0 and K % 8 == 0 and _tma_rows(x, w)):
+        return fused.swiglu(linear(x, w))
+    ws = torch.empty((splits * M, N), dtype=torch.float32, device=x.device)
+    out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
+    rc = _lib.kernels().b200_gemm_bf16_splitk_swiglu(
+        _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), _lib.ptr(ws), ctypes.c_int(M), ctypes.c_int(N // 2), ctypes.c_int(K),
+        ctypes.c_longlong(x.stride(0)), ctypes.c_longlong(w.stride(0)), ctypes.c_int(splits), ctypes.c_int(int(chained)),
+        _lib.stream_ptr())
+    _lib.check(rc, "b200_gemm_bf16_splitk_swiglu")
+    _lib.count_launch(2)
+    return out
 
 
 class _Linear(torch.autograd.Function):

@@ -443,7 +443,7 @@ def gated_linear(x: torch.Tensor, gate_up: torch.Tensor, act: GatedAct) -> torch
     lib = _lib.kernels()
     if x.dtype == torch.bfloat16 and I % 8 == 0 and H % 8 == 0 and _tma_rows(x, gate_up):
         splits = _splitk_plan(T, 2 * I, H)
-        ws = torch.empty((splits * -(-T // 128) * 128, 2 * I), dtype=torch.float32, device=x.device) if splits else None
+        ws = torch.empty((splits * T, 2 * I), dtype=torch.float32, device=x.device) if splits else None
         _lib.check(lib.b200_gemm_bf16_glu(p(x), p(gate_up), p(out), p(ws), c(T), c(I), c(H), ll(x.stride(0)),
                                           ll(gate_up.stride(0)), c(splits), *glu, _lib.stream_ptr()), "b200_gemm_bf16_glu")
         _lib.count_launch(2 if splits else 1)

@@ -59,8 +59,9 @@ def paged_decode_ref(q, k_cache, v_cache, block_table, seq_lens, scale=None):
 
 
 def paged_decode(q, k_cache, v_cache, block_table, seq_lens, scale=None, nsplit: int | None = None,
-                 max_seq_len: int | None = None):
-    """One query token per sequence attending to its paged cache (GQA)."""
+                 max_seq_len: int | None = None, chained: bool = False):
+    """One query token per sequence attending to its paged cache (GQA). ``chained``: launched as a programmatic dependent
+    of the kernel before it (a decode step's kernels, whose start-up then overlaps)."""
     B, Hq, D = q.shape
     scale = scale or 1.0 / math.sqrt(D)
     nb, Hkv, bs, _ = k_cache.shape
@@ -98,7 +99,7 @@ def paged_decode(q, k_cache, v_cache, block_table, seq_lens, scale=None, nsplit:
                                _lib.ptr(o_part), _lib.ptr(ml_part), ctypes.c_int(B),
                                ctypes.c_int(Hq), ctypes.c_int(Hkv), ctypes.c_int(D),
                                ctypes.c_int(bs), ctypes.c_int(nb), ctypes.c_int(block_table.shape[1]),
-                               ctypes.c_int(nsplit), ctypes.c_float(scale), _lib.stream_ptr())
+                               ctypes.c_int(nsplit), ctypes.c_float(scale), ctypes.c_int(int(chained)), _lib.stream_ptr())
     _lib.check(rc, "b200_paged_decode")
     _lib.count_launch(2 if nsplit > 1 else 1)
     return out
