@@ -3,7 +3,8 @@
 // A single CTA's 128 x 256 tile takes in 48 KB per 64-wide reduction block, 94 bytes per cycle of its products: more than L2
 // hands an SM. Here each CTA of the pair loads its own 128 rows of A and half of B's 256 (32 KB), the even CTA issues
 // products that read both, and each CTA's TMEM collects its own 128 rows. Policies, operand majors and epilogue are those of
-// the single-CTA kernel (a policy sees 128-row blocks; the optional grouped members are not supported).
+// the single-CTA kernel (a policy sees 128-row blocks; the optional grouped members are not supported). 16384 x 12288 x 2048:
+// 1519 TFLOP/s forward and 1540 dgrad, against 1102 to 1290 and 1307 to 1457 on single SMs.
 //
 // Barriers: `full` and `tempty` live in the even CTA (loads of both CTAs complete on it, epilogue warps of both arrive on it),
 // `empty` and `tfull` in each CTA (the even CTA's commits arrive in both). Every wait is bounded, as in gemm_core.cuh. No load

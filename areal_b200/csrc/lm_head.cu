@@ -17,6 +17,7 @@
 // Replaces the reference's chunked log_softmax over materialised logits and its
 // 3-4 all-reduces (areal/utils/functional/vocab_parallel.py:84-372).
 #include "common/gemm_core.cuh"
+#include "common/gemm_pair.cuh"
 #include "common/host_utils.h"
 #include "common/io.cuh"
 
@@ -374,6 +375,21 @@ __global__ void lm_sample_combine_kernel(const LmSampleRec* __restrict__ partial
   if (blockIdx.x == 0 && threadIdx.x == 0) rng[1] += 1ull;
 }
 
+// Work of the training-side products: 256-row tiles on pairs of SMs, or single ones for up to 128 rows (where half a pair's
+// rows would be padding).
+static bool lm_pairs(int T) { return T > 128; }
+
+template <class Epi>
+static int launch_lm_pair(const void* X, const void* W, int T, int V, int H, long long ldx, long long ldw,
+                          const Epi& epi, cudaStream_t stream) {
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_2d(&tmA, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, H, ldx * 2, kBM, 64);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, V, H, ldw * 2, PairCfg::kBN / 2, 64);
+  if (rc) return rc;
+  return launch_pair_epi<false, false>(tmA, tmB, T, V, H, epi, stream);
+}
+
 template <class Epi>
 static int launch_lm(const void* X, const void* W, int T, int V, int H, long long ldx,
                      long long ldw, const Epi& epi, long long work_items, cudaStream_t stream) {
@@ -404,16 +420,25 @@ static int launch_lm(const void* X, const void* W, int T, int V, int H, long lon
 
 extern "C" {
 
-// Number of vocab splits the forward uses for (T, V): enough work items to
-// fill the SMs without making the partial buffer large.
+// Number of vocab splits the forward uses for (T, V): the split length (in 256-column blocks) at which the busiest CTA (or pair)
+// has the fewest tiles, in at most 64 splits; ties go to fewer splits. 8192 rows of a 151936-token vocabulary: 23 splits, 99% of the
+// SMs' time, where "twice as many items as SMs" left a third round 16% full.
 int b200_lm_head_nsplit(int T, int V) {
-  const int tiles_m = (T + 127) / 128;
   const int tiles_n = (V + 255) / 256;
-  int want = (2 * b200::sm_count() + tiles_m - 1) / tiles_m;
-  if (want < 1) want = 1;
-  if (want > tiles_n) want = tiles_n;
-  const int nb_per = (tiles_n + want - 1) / want;
-  return (tiles_n + nb_per - 1) / nb_per;
+  const bool pairs = b200::lm_pairs(T);
+  const long long tiles_m = pairs ? (T + 255) / 256 : (T + 127) / 128, units = pairs ? b200::sm_count() / 2 : b200::sm_count();
+  long long best_cost = -1;
+  int best = 1;
+  for (int nb = tiles_n; nb >= 1; --nb) {
+    const int nsplit = (tiles_n + nb - 1) / nb;
+    if (nsplit > 64) break;
+    const long long cost = ((nsplit * tiles_m + units - 1) / units) * nb;
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = nsplit;
+    }
+  }
+  return best;
 }
 
 // partials: fp32 [nsplit, T, 4] with nsplit = b200_lm_head_nsplit(T, V).
@@ -428,6 +453,7 @@ int b200_lm_head_stats(const void* X, const void* W, const int* labels, float* p
   const int nb_per = (tiles_n + nsplit - 1) / nsplit;
   LmStatsEpi epi{partials, {}, 0, 0, labels, T, V, vocab_start, nb_per, nsplit, inv_temp,
                  soft_cap(softcap)};
+  if (lm_pairs(T)) return launch_lm_pair(X, W, T, V, H, ldx, ldw, epi, stream);
   return launch_lm(X, W, T, V, H, ldx, ldw, epi, static_cast<long long>(tiles_m) * nsplit,
                    stream);
 }
@@ -449,6 +475,7 @@ int b200_lm_head_stats_peers(const void* X, const void* W, const int* labels, vo
   LmStatsEpi epi{nullptr, {}, n_peers, rank * nsplit, labels, T, V, vocab_start, nb_per, nsplit, inv_temp,
                  soft_cap(softcap)};
   for (int p = 0; p < n_peers; ++p) epi.peers[p] = reinterpret_cast<float*>(peer_partials[p]);
+  if (lm_pairs(T)) return launch_lm_pair(X, W, T, V, H, ldx, ldw, epi, stream);
   return launch_lm(X, W, T, V, H, ldx, ldw, epi, static_cast<long long>(tiles_m) * nsplit, stream);
 }
 
@@ -519,6 +546,7 @@ int b200_lm_head_dlogits(const void* X, const void* W, const int* labels, const 
   if (T == 0 || V == 0) return 0;
   LmDlogitsEpi epi{reinterpret_cast<__nv_bfloat16*>(dz), labels, g_logp, g_ent, logz, ey, ldz, T, V,
                    vocab_start, inv_temp, soft_cap(softcap)};
+  if (lm_pairs(T)) return launch_lm_pair(X, W, T, V, H, ldx, ldw, epi, stream);
   const long long tiles = static_cast<long long>((T + 127) / 128) * ((V + 255) / 256);
   return launch_lm(X, W, T, V, H, ldx, ldw, epi, tiles, stream);
 }

@@ -104,12 +104,7 @@ def gemm(
             _lib.count_launch(2)
             return out
     if bn == 0:
-        bn = 256 if N > 128 else 128
-        if bn == 256:
-            # Prefer 128-wide tiles when 256-wide ones would leave most SMs idle.
-            tiles256 = -(-M // 128) * -(-N // 256)
-            if tiles256 < 100:
-                bn = 128
+        bn = _tile_plan(M, N)
     lib = _lib.kernels()
     fn = lib.b200_gemm_bf16
     fn.restype = ctypes.c_int
@@ -125,6 +120,17 @@ def gemm(
     _lib.check(rc, "b200_gemm_bf16")
     _lib.count_launch()
     return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _tile_plan(M: int, N: int) -> int:
+    """Tile of a product that is not split: 512 (256 x 256 on a pair of SMs), 256 or 128 (128 rows by so many columns on one).
+    Whole rounds of tiles over the SMs, times what a tile takes. Forward / dgrad / wgrad of 16384 x 4096 x 2048 in TFLOP/s: 1495 / 1514 /
+    1324 on pairs, 1318 / 1397 / 1251 with 256 columns, 1162 / 1239 / 1108 with 128; of 2600 x 2048 x 2048, where pairs leave
+    40% of their second round empty, 734 / 757 / 589, 757 / 757 / 620 and 880 / 880 / 662."""
+    cost = {512: 1.0 * -(-(-(-M // 256) * -(-N // 256)) // 74), 256: 1.1 * -(-(-(-M // 128) * -(-N // 256)) // 148),
+            128: 0.63 * -(-(-(-M // 128) * -(-N // 128)) // 148)}
+    return min(cost, key=cost.get)
 
 
 @functools.lru_cache(maxsize=4096)
