@@ -37,6 +37,11 @@ constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kGemmThreads = 192;
 
+// A policy may ask for shared memory of its own: kWarpSmem bytes (a multiple of 1024) for each of the four epilogue warps,
+// whose address `bind` puts into its state.
+template <class E> __host__ __device__ constexpr auto epi_warp_smem(int) -> decltype(E::kWarpSmem) { return E::kWarpSmem; }
+template <class E> __host__ __device__ constexpr int epi_warp_smem(long) { return 0; }
+
 template <int BN>
 struct GemmCfg {
   // 32- and 64-wide tiles are for products that stream a weight past a few rows: more stages, the same bytes in flight
@@ -95,7 +100,7 @@ template <class E> __device__ constexpr bool epi_chained(long) { return false; }
 template <int BN, bool A_MN, bool B_MN, class Epi>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    int M, int N, int K, Epi epi, int* status) {
+                    int M, int N, int K, const __grid_constant__ Epi epi, int* status) {
   using Cfg = GemmCfg<BN>;
   constexpr int STAGES = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -103,7 +108,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * Cfg::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes);
+  uint8_t* smem_epi = smem + STAGES * Cfg::kStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_epi + 4 * epi_warp_smem<Epi>(0));
   uint64_t* full = bars;
   uint64_t* empty = bars + STAGES;
   uint64_t* tfull = bars + 2 * STAGES;
@@ -274,6 +280,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ---------------------------------------------------------- epilogue --
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32)
     typename Epi::State st;
+    if constexpr (epi_warp_smem<Epi>(0) > 0) epi.bind(st, smem_epi + quarter * epi_warp_smem<Epi>(0));
     bool ok = true;
     for (int it = 0; ok; ++it) {
       int m_blk, n_blk;

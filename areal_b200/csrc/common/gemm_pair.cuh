@@ -72,7 +72,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 template <bool A_MN, bool B_MN, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
-                 Epi epi, int* status) {
+                 const __grid_constant__ Epi epi, int* status) {
   using Cfg = PairCfg;
   constexpr int STAGES = Cfg::kStages, BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
@@ -81,7 +81,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * Cfg::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes);
+  uint8_t* smem_epi = smem + STAGES * Cfg::kStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_epi + 4 * epi_warp_smem<Epi>(0));
   uint64_t* full = bars;
   uint64_t* empty = bars + STAGES;
   uint64_t* tfull = bars + 2 * STAGES;
@@ -230,6 +231,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ---------------------------------------------------------- epilogue --
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32)
     typename Epi::State st;
+    if constexpr (epi_warp_smem<Epi>(0) > 0) epi.bind(st, smem_epi + quarter * epi_warp_smem<Epi>(0));
     bool ok = true;
     for (int it = 0; ok; ++it) {
       int mp, n_blk;
@@ -280,9 +282,10 @@ template <bool A_MN, bool B_MN, class Epi>
 int launch_pair_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, int M, int N, int K, const Epi& epi,
                     cudaStream_t stream) {
   auto kern = gemm_pair_kernel<A_MN, B_MN, Epi>;
+  constexpr int smem = PairCfg::kSmemBytes + 4 * epi_warp_smem<Epi>(0);
   static bool attr_set = false;
   if (!attr_set) {
-    B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kSmemBytes));
+    B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set = true;
   }
   const long long tiles = static_cast<long long>((M + 2 * kBM - 1) / (2 * kBM)) * ((N + PairCfg::kBN - 1) / PairCfg::kBN);
@@ -291,7 +294,7 @@ int launch_pair_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, int M, int N
   if (grid <= 0) return 0;
   int* status = device_status_word();
   if (!status) return -3;
-  kern<<<grid, kGemmThreads, PairCfg::kSmemBytes, stream>>>(tmA, tmB, M, N, K, epi, status);
+  kern<<<grid, kGemmThreads, smem, stream>>>(tmA, tmB, M, N, K, epi, status);
   B200_CHECK(cudaGetLastError());
   return 0;
 }
