@@ -39,6 +39,18 @@ def _gemm_ref(a, b, a_mn, b_mn, bias, out_dtype, out, accumulate):
     return c.to(out_dtype)
 
 
+def _tma_operand(t: torch.Tensor) -> torch.Tensor:
+    """``t`` with unit inner stride and a 16-byte aligned base and pitch, as TMA needs them. The extents stay what they are: a
+    reduction rounded up beyond one operand's rows would read what lies behind it, and zeros times that need not be zero."""
+    if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0:
+        return t
+    n = t.shape[1]
+    if n % 8:
+        return torch.nn.functional.pad(t, (0, -n % 8))[:, :n]
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -63,10 +75,7 @@ def gemm(
         return _gemm_ref(a, b, a_mn, b_mn, bias, out_dtype, out, accumulate)
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "bf16 operands required"
     assert a.dim() == 2 and b.dim() == 2
-    if a.stride(1) != 1 or (a.stride(0) % 8) or (a.data_ptr() % 16):
-        a = a.contiguous()
-    if b.stride(1) != 1 or (b.stride(0) % 8) or (b.data_ptr() % 16):
-        b = b.contiguous()
+    a, b = _tma_operand(a), _tma_operand(b)
     if a_mn:
         K, M = a.shape
     else:
@@ -81,18 +90,10 @@ def gemm(
         accumulate = False
     assert out.shape == (M, N) and out.stride(1) == 1
     assert out.dtype in (torch.bfloat16, torch.float32)
-    # TMA needs 16-byte aligned pitches: pad the contiguous extent when it is not.
-    need_pad = (a.shape[1] % 8) or (b.shape[1] % 8)
-    if need_pad:
-        def pad(t):
-            p = (-t.shape[1]) % 8
-            return torch.nn.functional.pad(t, (0, p)) if p else t
-        a, b = pad(a), pad(b)
-        if not a_mn:
-            K = a.shape[1]
+    ragged = (a.shape[1] % 8) or (b.shape[1] % 8)
     # skinny products (decode steps): too few output tiles for 148 SMs ⇒ split the K extent
     if (bn == 0 and not a_mn and not b_mn and not accumulate and out.dtype == torch.bfloat16 and out.stride(0) % 4 == 0
-            and not need_pad):
+            and not ragged):
         splits = _splitk_plan(M, N, K)
         if splits:
             ws = torch.empty((splits * M, N), dtype=torch.float32, device=a.device)
