@@ -137,11 +137,11 @@ def _tile_plan(M: int, N: int) -> int:
 @functools.lru_cache(maxsize=4096)
 def _splitk_plan(M: int, N: int, K: int) -> int:
     """Number of K slices of the skinny path for this shape (0: not a shape for it). The kernel walks items of 128 weight
-    rows by a K slice, one CTA per SM, so a pass takes ``rounds of items * (reduction blocks of an item + its start)``; what is saved
-    there by more slices is paid for with partial sums that are written and read back. Up to 128 rows the two are weighed in bytes
-    (the sums at half price: they stay in L2). With more rows the sums of many slices cost more than they save (a decode step of
-    256 rows of Qwen3-1.7B: 8.45 ms by that rule, 7.49 ms with slices for a single round of items), and a product with as
-    many tiles as half the SMs is not split."""
+    rows by a K slice, one CTA per SM, so a pass takes ``rounds of items * (reduction blocks of an item + its start)``, and each
+    slice makes the reduction behind it longer. Up to 128 rows this is weighed in bytes against the partial sums that are
+    written and read back (at half price: they stay in L2). One sequence of Qwen3-1.7B: 1.48 ms a step when slices cost nothing but
+    their sums, 1.43 ms so. With more rows the sums of many slices cost more than they save (256 rows: 8.45 ms by that
+    rule, 7.49 ms with slices for a single round of items), and a product with as many tiles as half the SMs is not split."""
     if M > 512 or N % 4 or K < 1024:
         return 0
     tiles, blocks = -(-M // 128) * -(-N // 128), -(-K // 64)
@@ -149,8 +149,9 @@ def _splitk_plan(M: int, N: int, K: int) -> int:
         splits = min(8, 148 // tiles, K // 256)
     else:
         rows = 32 if M <= 32 else 64 if M <= 64 else 128
+        step = 148 * (128 + rows / 2) * 128  # bytes that all CTAs load per reduction block
         splits = min(range(1, min(16, blocks // 2) + 1),
-                     key=lambda s: -(-tiles * s // 148) * (-(-blocks // s) + 2) * 148 * (128 + rows / 2) * 128 + 4 * s * M * N)
+                     key=lambda s: (-(-tiles * s // 148) * (-(-blocks // s) + 2) + 2 * s) * step + 4 * s * M * N)
     return splits if splits >= 2 else 0
 
 
