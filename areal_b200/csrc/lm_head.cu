@@ -139,7 +139,7 @@ __global__ void lm_combine_kernel(const float* __restrict__ partials, int nparts
   }
   const float lz = M + logf(L);
   const float e = SX / L;
-  if (logp) logp[row] = t - lz;
+  if (logp) logp[row] = (t - M) - logf(L);  // in this order: near the maximum nothing cancels
   if (entropy) entropy[row] = lz - e;
   if (logz) logz[row] = lz;
   if (ey) ey[row] = e;
@@ -328,6 +328,99 @@ struct LmSampleEpi {
   }
 };
 
+// The same head for up to 32 rows: the vocabulary is the 128-row side of the tile and the rows are its columns, so a thread owns one
+// vocabulary entry of every row. With the rows on the 128-row side one row left one thread to draw all of a tile's noise: 171
+// us for one row and 242 us for 16 rows of a 4096-wide model, where the weight's read takes 95 and 190 us; now 96 and 195 us. A thread keeps its
+// records over the CTA's tiles; lanes merge at the end, one part per epilogue warp. Noise and draws are those of LmSampleEpi.
+template <int NB>
+struct LmSampleThinEpi {
+  LmSampleRec* partials;      // [4 * CTAs, T]
+  int* part_idx;              // [4 * CTAs, T]
+  const float* temperature;   // [T]
+  const unsigned long long* rng;
+  int T, V;                   // T <= NB
+  SoftCap cap;
+  struct State {
+    float m[NB], l[NB], best[NB], bx[NB];
+    int bi[NB];
+    bool last;
+  };
+  __device__ __forceinline__ bool tile(int cta, int ncta, int it, int tiles_v, int, int& v_blk, int& n_blk) const {
+    v_blk = it * ncta + cta;
+    n_blk = 0;
+    return v_blk < tiles_v;
+  }
+  __device__ __forceinline__ bool gate(int, int, volatile int*, int*) const { return true; }
+  __device__ __forceinline__ void begin(State& s, int v_blk, int, int) const {
+    if (v_blk < static_cast<int>(gridDim.x)) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        s.m[b] = s.best[b] = -INFINITY;
+        s.l[b] = s.bx[b] = 0.f;
+        s.bi[b] = 0x7fffffff;
+      }
+    }
+    s.last = (v_blk + static_cast<int>(gridDim.x)) * kBM >= V;
+  }
+  __device__ __forceinline__ void chunk(State& s, int col, int, const float (&v)[32]) const {
+    if (col >= V) return;
+    float z[32];
+    cap.apply(v, z);
+    const unsigned long long seed = rng[0], step = rng[1];
+    const uint2 key = make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (b >= T) break;
+      const float t = temperature[b];
+      const float x = t > 0.f ? z[b] * (1.f / t) : z[b];
+      const float m = fmaxf(s.m[b], x);
+      if (m != -INFINITY) s.l[b] = s.l[b] * __expf(s.m[b] - m) + __expf(x - m);
+      s.m[b] = m;
+      float score = x;
+      if (t > 0.f) {
+        const uint4 q = philox4x32_7(make_uint4(static_cast<uint32_t>(col >> 2), static_cast<uint32_t>(b),
+                                                static_cast<uint32_t>(step), static_cast<uint32_t>(step >> 32)), key);
+        const uint32_t lo = col & 1 ? q.y : q.x, hi = col & 1 ? q.w : q.z;
+        score += gumbel_from_bits(col & 2 ? hi : lo);
+      }
+      if (score > s.best[b]) {  // strict: the smallest index wins a tie
+        s.best[b] = score;
+        s.bx[b] = x;
+        s.bi[b] = col;
+      }
+    }
+  }
+  __device__ __forceinline__ void end(State& s, int, int, int) const {
+    if (!s.last) return;
+    const int lane = threadIdx.x & 31;
+    const long long part = blockIdx.x * 4 + ((threadIdx.x >> 5) & 3);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (b >= T) break;
+      float m = s.m[b], l = s.l[b], best = s.best[b], bx = s.bx[b];
+      int bi = s.bi[b];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+        const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, bx, o);
+        const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+        const float mn = fmaxf(m, m2);
+        if (mn != -INFINITY) l = l * __expf(m - mn) + l2 * __expf(m2 - mn);
+        m = mn;
+        if (b2 > best || (b2 == best && i2 < bi)) {
+          best = b2;
+          bx = x2;
+          bi = i2;
+        }
+      }
+      if (lane == 0) {
+        partials[part * T + b] = LmSampleRec{m, l, best, bx};
+        part_idx[part * T + b] = bi;
+      }
+    }
+  }
+};
+
 // One warp per row: the lanes stride over the vocab splits, then merge (max, sum-exp) pairs and the best
 // perturbed score by shuffles (ties go to the lower split, i.e. the smaller token id).
 __global__ void lm_sample_combine_kernel(const LmSampleRec* __restrict__ partials, const int* __restrict__ part_idx,
@@ -337,7 +430,7 @@ __global__ void lm_sample_combine_kernel(const LmSampleRec* __restrict__ partial
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row < T) {
     float m = -INFINITY, l = 0.f, best = -INFINITY, bx = 0.f;
-    int bp = 0x7fffffff;
+    int bi = 0x7fffffff;  // the token of the best score; the smaller one of a tie
     for (int p = lane; p < nparts; p += 32) {
       const LmSampleRec r = partials[static_cast<long long>(p) * T + row];
       if (r.m != -INFINITY) {
@@ -345,30 +438,31 @@ __global__ void lm_sample_combine_kernel(const LmSampleRec* __restrict__ partial
         l = l * ((m == -INFINITY) ? 0.f : __expf(m - mn)) + r.l * __expf(r.m - mn);
         m = mn;
       }
-      if (r.best > best) {
+      const int i = part_idx[static_cast<long long>(p) * T + row];
+      if (r.best > best || (r.best == best && i < bi)) {
         best = r.best;
         bx = r.bx;
-        bp = p;
+        bi = i;
       }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
       const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, bx, o);
-      const int p2 = __shfl_xor_sync(0xffffffffu, bp, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
       const float mn = fmaxf(m, m2);
       const float s1 = (m == -INFINITY) ? 0.f : __expf(m - mn), s2 = (m2 == -INFINITY) ? 0.f : __expf(m2 - mn);
       l = l * s1 + l2 * s2;
       m = mn;
-      if (b2 > best || (b2 == best && p2 < bp)) {
+      if (b2 > best || (b2 == best && i2 < bi)) {
         best = b2;
         bx = x2;
-        bp = p2;
+        bi = i2;
       }
     }
     if (lane == 0) {
-      tokens[row] = (bp == 0x7fffffff) ? 0 : part_idx[static_cast<long long>(bp) * T + row];
-      logprobs[row] = bx - (m + logf(l));
+      tokens[row] = bi == 0x7fffffff ? 0 : bi;
+      logprobs[row] = (bx - m) - logf(l);  // in this order: near the maximum nothing cancels
     }
   }
   // every block of the GEMM that read the counter has finished (stream order): advance it for the next step
@@ -412,6 +506,35 @@ static int launch_lm(const void* X, const void* W, int T, int V, int H, long lon
   int* status = device_status_word();
   if (!status) return -3;
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(tmA, tmB, T, V, H, epi, status);
+  B200_CHECK(cudaGetLastError());
+  return 0;
+}
+
+// LmSampleThinEpi: the vocabulary on the 128-row side, up to 32 rows on the other.
+constexpr int kThinRows = 32;
+
+template <int NB>
+static int launch_lm_thin(const void* X, const void* W, const float* temperature, LmSampleRec* partials, int* part_idx,
+                          const unsigned long long* rng, int B, int V, int H, long long ldx, long long ldw, SoftCap cap,
+                          cudaStream_t stream) {
+  constexpr int BN = kThinRows;
+  using Cfg = GemmCfg<BN>;
+  CUtensorMap tmW, tmX;
+  int rc = make_tmap_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, V, H, ldw * 2, kBM, 64);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, H, ldx * 2, BN, 64);
+  if (rc) return rc;
+  const LmSampleThinEpi<NB> epi{partials, part_idx, temperature, rng, B, V, cap};
+  auto kern = gemm_tcgen05_kernel<BN, false, false, LmSampleThinEpi<NB>>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    attr_set = true;
+  }
+  const int tiles = (V + kBM - 1) / kBM, grid = tiles < sm_count() ? tiles : sm_count();
+  int* status = device_status_word();
+  if (!status) return -3;
+  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(tmW, tmX, V, B, H, epi, status);
   B200_CHECK(cudaGetLastError());
   return 0;
 }
@@ -499,7 +622,12 @@ int b200_lm_head_sample_nb_per(int B, int V) {
   return best;
 }
 
+// Parts per row of the sampling head: vocab splits, or (up to 32 rows) the epilogue warps of all CTAs.
 int b200_lm_head_sample_nsplit(int B, int V) {
+  if (B <= b200::kThinRows) {
+    const int tiles = (V + 127) / 128;
+    return 4 * (tiles < b200::sm_count() ? tiles : b200::sm_count());
+  }
   const int tiles_n = (V + 255) / 256;
   const int nb = b200_lm_head_sample_nb_per(B, V);
   return (tiles_n + nb - 1) / nb;
@@ -514,12 +642,17 @@ int b200_lm_head_sample(const void* X, const void* W, const float* temperature, 
                         long long ldx, long long ldw, float softcap, cudaStream_t stream) {
   using namespace b200;
   if (B == 0 || V == 0) return 0;
-  const int tiles_m = (B + 127) / 128;
-  const int nb_per = b200_lm_head_sample_nb_per(B, V);
   const int nsplit = b200_lm_head_sample_nsplit(B, V);
-  LmSampleEpi epi{reinterpret_cast<LmSampleRec*>(partials), part_idx, temperature, rng, B, V, nb_per, nsplit,
-                  soft_cap(softcap)};
-  int rc = launch_lm(X, W, B, V, H, ldx, ldw, epi, static_cast<long long>(tiles_m) * nsplit, stream);
+  auto* recs = reinterpret_cast<LmSampleRec*>(partials);
+  int rc;
+  if (B <= kThinRows) {
+    auto thin = B <= 8 ? launch_lm_thin<8> : B <= 16 ? launch_lm_thin<16> : launch_lm_thin<32>;
+    rc = thin(X, W, temperature, recs, part_idx, rng, B, V, H, ldx, ldw, soft_cap(softcap), stream);
+  } else {
+    const int tiles_m = (B + 127) / 128, nb_per = b200_lm_head_sample_nb_per(B, V);
+    const LmSampleEpi epi{recs, part_idx, temperature, rng, B, V, nb_per, nsplit, soft_cap(softcap)};
+    rc = launch_lm(X, W, B, V, H, ldx, ldw, epi, static_cast<long long>(tiles_m) * nsplit, stream);
+  }
   if (rc) return rc;
   lm_sample_combine_kernel<<<(B + 3) / 4, 128, 0, stream>>>(reinterpret_cast<const LmSampleRec*>(partials),
                                                                 part_idx, nsplit, B, tokens, logprobs, rng);

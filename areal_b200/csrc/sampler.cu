@@ -234,7 +234,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V,
   });
   const float M = block_max(mx, s.fpart);
   const float Z = block_add(mx == -INFINITY ? se : se * __expf(mx - M), s.fpart);
-  const float logZ = M + logf(Z);
+  const float logZ = logf(Z);  // of the shifted logits: near the maximum nothing cancels
   // the first index of the maximum: a thread's vectors come in rising order, the block's minimum decides
   int best = 0x7fffffff;
   if (mx == M && mx > -INFINITY)
@@ -255,7 +255,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V,
   if (greedy) {
     if (tid == 0) {
       tokens[b] = best;
-      logprobs[b] = x[best] * inv_t - logZ;
+      logprobs[b] = (x[best] * inv_t - M) - logZ;
     }
     return;
   }
@@ -442,7 +442,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V,
     // numerical corner (target == total): the most likely token
     const int pick = s.pick >= 0 ? s.pick : best;
     tokens[b] = pick;
-    logprobs[b] = x[pick] * inv_t - logZ;
+    logprobs[b] = (x[pick] * inv_t - M) - logZ;
   }
 }
 
