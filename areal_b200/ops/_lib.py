@@ -60,19 +60,46 @@ def use_cuda_kernels(*tensors: torch.Tensor) -> bool:
     routes CUDA tensors to the PyTorch reference instead (used by tests that
     compare the two on the same device).
     """
-    if not tensors or not all(t.is_cuda for t in tensors if t is not None):
+    if not tensors:
         return False
+    for t in tensors:
+        if t is not None and not t.is_cuda:
+            return False
     if os.environ.get("AREAL_B200_FORCE_TORCH") == "1":
         return False
-    lib = kernels()  # raises loudly if the library is missing on a GPU box
-    rc = lib.b200_ensure_device(ctypes.c_int(tensors[0].device.index or 0))
+    # raises loudly if the library is missing on a GPU box
+    rc = bind("b200_ensure_device", "i")(tensors[0].get_device())
     if rc != 0:
         raise RuntimeError(f"b200_ensure_device failed with code {rc}")
     return True
 
 
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
+
+
+@functools.lru_cache(maxsize=None)
+def bind(name: str, signature: str):
+    """The kernel library's function ``name`` with its argument types set once (``p``ointer, ``i``nt, ``l``ong long,
+    ``f``loat; blanks are ignored), so that calls pass plain numbers: building a ctypes object per argument and call took longer
+    than the launch itself."""
+    fn = getattr(kernels(), name)
+    fn.argtypes = [_CTYPES[c] for c in signature if c != " "]
+    fn.restype = ctypes.c_int
+    return fn
+
+
+def stream_raw() -> int:
+    """Handle of the current stream of the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(stream_raw())
+
+
+def addr(t: torch.Tensor | None) -> int | None:
+    """A tensor's address for a bound function (None: null)."""
+    return None if t is None else t.data_ptr()
 
 
 def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:

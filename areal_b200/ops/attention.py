@@ -10,7 +10,6 @@ The work lists (one record per 128-row tile) are built on the host from
 
 from __future__ import annotations
 
-import ctypes
 import math
 
 import numpy as np
@@ -106,13 +105,9 @@ def _fwd_cuda(q, k, v, meta: VarlenMeta, scale):
     assert k.stride(2) == 1 and k.stride(1) == D and v.stride(2) == 1 and v.stride(1) == D
     o = torch.empty_like(q)
     lse = torch.empty((Hq, T), dtype=torch.float32, device=q.device)
-    fn = _lib.kernels().b200_attn_fwd
-    fn.restype = ctypes.c_int
-    rc = fn(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse),
-            _lib.ptr(meta.fwd_tiles), ctypes.c_int(meta.n_fwd), ctypes.c_int(T),
-            ctypes.c_int(Hq), ctypes.c_int(Hkv), ctypes.c_longlong(q.stride(0)),
-            ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(v.stride(0)),
-            ctypes.c_float(scale), _lib.stream_ptr())
+    rc = _lib.bind("b200_attn_fwd", "pppppp iiii lll f p")(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), meta.fwd_tiles.data_ptr(), meta.n_fwd, T, Hq,
+        Hkv, q.stride(0), k.stride(0), v.stride(0), scale, _lib.stream_raw())
     _lib.check(rc, "b200_attn_fwd")
     _lib.count_launch()
     return o, lse
@@ -127,14 +122,10 @@ def _bwd_cuda(q, k, v, o, do, lse, meta: VarlenMeta, scale, dk_out=None, dv_out=
     dq = torch.empty_like(q)
     dk = dk_out if dk_out is not None else torch.empty((T, Hkv, D), dtype=q.dtype, device=q.device)
     dv = dv_out if dv_out is not None else torch.empty((T, Hkv, D), dtype=q.dtype, device=q.device)
-    fn = _lib.kernels().b200_attn_bwd
-    fn.restype = ctypes.c_int
-    rc = fn(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(do), _lib.ptr(lse),
-            _lib.ptr(delta), _lib.ptr(dq_acc), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv),
-            _lib.ptr(meta.bwd_tiles), ctypes.c_int(meta.n_bwd), ctypes.c_int(T),
-            ctypes.c_int(Hq), ctypes.c_int(Hkv), ctypes.c_longlong(k.stride(0)),
-            ctypes.c_longlong(v.stride(0)), ctypes.c_longlong(dk.stride(0)),
-            ctypes.c_longlong(dv.stride(0)), ctypes.c_float(scale), _lib.stream_ptr())
+    rc = _lib.bind("b200_attn_bwd", "pppppppppppp iiii llll f p")(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+        dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), meta.bwd_tiles.data_ptr(), meta.n_bwd, T, Hq, Hkv,
+        k.stride(0), v.stride(0), dk.stride(0), dv.stride(0), scale, _lib.stream_raw())
     _lib.check(rc, "b200_attn_bwd")
     _lib.count_launch(3)
     return dq, dk, dv

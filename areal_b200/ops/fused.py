@@ -37,17 +37,14 @@ class _RMSNorm(torch.autograd.Function):
         T = x2.shape[0]
         y = torch.empty_like(x2)
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-        lib = _lib.kernels()
-        lib.b200_rmsnorm_fwd.restype = ctypes.c_int
         if residual is not None:
             r2 = residual.reshape(-1, H)
             r2 = r2 if r2.is_contiguous() else r2.contiguous()
             h = torch.empty_like(x2)
         else:
             r2, h = None, None
-        rc = lib.b200_rmsnorm_fwd(_lib.ptr(x2), _lib.ptr(r2), _lib.ptr(w), _lib.ptr(y), _lib.ptr(h),
-                                  _lib.ptr(rstd), ctypes.c_int(T), ctypes.c_int(H),
-                                  ctypes.c_float(eps), _lib.stream_ptr())
+        rc = _lib.bind("b200_rmsnorm_fwd", "pppppp iif p")(x2.data_ptr(), _lib.addr(r2), w.data_ptr(), y.data_ptr(),
+                                                           _lib.addr(h), rstd.data_ptr(), T, H, eps, _lib.stream_raw())
         _lib.check(rc, "b200_rmsnorm_fwd")
         _lib.count_launch()
         ctx.save_for_backward(h if h is not None else x2, w, rstd)
@@ -67,17 +64,13 @@ class _RMSNorm(torch.autograd.Function):
         if ctx.has_res and dh is not None:
             dres = dh.reshape(T, H)
             dres = dres if dres.is_contiguous() else dres.contiguous()
-        lib = _lib.kernels()
-        lib.b200_rmsnorm_bwd_blocks.restype = ctypes.c_int
-        nb = lib.b200_rmsnorm_bwd_blocks(ctypes.c_int(T))
+        nb = _lib.bind("b200_rmsnorm_bwd_blocks", "i")(T)
         partial = torch.empty((nb, H), dtype=torch.float32, device=xin.device)
         dw = torch.empty(H, dtype=torch.float32, device=xin.device)
         dx = torch.empty_like(xin)
-        lib.b200_rmsnorm_bwd.restype = ctypes.c_int
-        rc = lib.b200_rmsnorm_bwd(_lib.ptr(dy2), _lib.ptr(xin), _lib.ptr(w), _lib.ptr(rstd),
-                                  _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(partial), _lib.ptr(dw),
-                                  ctypes.c_int(0), ctypes.c_int(T), ctypes.c_int(H),
-                                  _lib.stream_ptr())
+        rc = _lib.bind("b200_rmsnorm_bwd", "pppppppp iii p")(
+            dy2.data_ptr(), xin.data_ptr(), w.data_ptr(), rstd.data_ptr(), _lib.addr(dres), dx.data_ptr(),
+            partial.data_ptr(), dw.data_ptr(), 0, T, H, _lib.stream_raw())
         _lib.check(rc, "b200_rmsnorm_bwd")
         _lib.count_launch(2)
         dxv = dx.view(ctx.shape)
@@ -186,13 +179,9 @@ class _QKNormRope(torch.autograd.Function):
                            device=qkv.device)
         if _lib.checked():
             _check_rope_args("qknorm_rope", qkv, qw, kw, cos, sin, pos, Hq, Hkv, D)
-        lib = _lib.kernels()
-        lib.b200_qknorm_rope_fwd.restype = ctypes.c_int
-        rc = lib.b200_qknorm_rope_fwd(_lib.ptr(qkv), _lib.ptr(qw), _lib.ptr(kw), _lib.ptr(cos),
-                                      _lib.ptr(sin), _lib.ptr(pos), _lib.ptr(q), _lib.ptr(k),
-                                      _lib.ptr(rstd), ctypes.c_int(T), ctypes.c_int(Hq),
-                                      ctypes.c_int(Hkv), ctypes.c_int(D), ctypes.c_float(eps),
-                                      ctypes.c_int(int(has_norm)), _lib.stream_ptr())
+        rc = _lib.bind("b200_qknorm_rope_fwd", "ppppppppp iiii f i p")(
+            qkv.data_ptr(), _lib.addr(qw), _lib.addr(kw), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), q.data_ptr(),
+            k.data_ptr(), rstd.data_ptr(), T, Hq, Hkv, D, eps, has_norm, _lib.stream_raw())
         _lib.check(rc, "b200_qknorm_rope_fwd")
         _lib.count_launch()
         v = qkv[:, (Hq + Hkv) * D:].view(T, Hkv, D)
@@ -208,15 +197,10 @@ class _QKNormRope(torch.autograd.Function):
         dqkv = torch.empty_like(qkv)
         dq, dk, dv = _lib.vec16(dq), _lib.vec16(dk), _lib.vec16(dv)
         dw = torch.zeros((2, D), dtype=torch.float32, device=qkv.device)  # of the q and the k norm
-        lib = _lib.kernels()
-        lib.b200_qknorm_rope_bwd.restype = ctypes.c_int
-        rc = lib.b200_qknorm_rope_bwd(_lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(qkv),
-                                      _lib.ptr(qw), _lib.ptr(kw), _lib.ptr(cos), _lib.ptr(sin),
-                                      _lib.ptr(pos), _lib.ptr(rstd), _lib.ptr(dqkv), _lib.ptr(dw[0]),
-                                      _lib.ptr(dw[1]),
-                                      ctypes.c_int(T), ctypes.c_int(Hq), ctypes.c_int(Hkv),
-                                      ctypes.c_int(D), ctypes.c_int(int(has_norm)),
-                                      _lib.stream_ptr())
+        rc = _lib.bind("b200_qknorm_rope_bwd", "ppppppppppppp iiiii p")(
+            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), qkv.data_ptr(), _lib.addr(qw), _lib.addr(kw), cos.data_ptr(),
+            sin.data_ptr(), pos.data_ptr(), rstd.data_ptr(), dqkv.data_ptr(), dw.data_ptr(), dw.data_ptr() + 4 * D, T, Hq,
+            Hkv, D, has_norm, _lib.stream_raw())
         _lib.check(rc, "b200_qknorm_rope_bwd")
         _lib.count_launch()
         if has_norm:
@@ -294,10 +278,7 @@ class _SwiGLU(torch.autograd.Function):
         g2 = gu.reshape(-1, 2 * inter)
         g2 = g2 if g2.is_contiguous() else g2.contiguous()
         out = torch.empty((g2.shape[0], inter), dtype=gu.dtype, device=gu.device)
-        lib = _lib.kernels()
-        lib.b200_swiglu_fwd.restype = ctypes.c_int
-        rc = lib.b200_swiglu_fwd(_lib.ptr(g2), _lib.ptr(out), ctypes.c_longlong(g2.shape[0]),
-                                 ctypes.c_int(inter), _lib.stream_ptr())
+        rc = _lib.bind("b200_swiglu_fwd", "pp l i p")(g2.data_ptr(), out.data_ptr(), g2.shape[0], inter, _lib.stream_raw())
         _lib.check(rc, "b200_swiglu_fwd")
         _lib.count_launch()
         ctx.save_for_backward(g2)
@@ -311,11 +292,8 @@ class _SwiGLU(torch.autograd.Function):
         dy2 = dy.reshape(-1, inter)
         dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
         dgu = torch.empty_like(g2)
-        lib = _lib.kernels()
-        lib.b200_swiglu_bwd.restype = ctypes.c_int
-        rc = lib.b200_swiglu_bwd(_lib.ptr(dy2), _lib.ptr(g2), _lib.ptr(dgu),
-                                 ctypes.c_longlong(g2.shape[0]), ctypes.c_int(inter),
-                                 _lib.stream_ptr())
+        rc = _lib.bind("b200_swiglu_bwd", "ppp l i p")(dy2.data_ptr(), g2.data_ptr(), dgu.data_ptr(), g2.shape[0], inter,
+                                                       _lib.stream_raw())
         _lib.check(rc, "b200_swiglu_bwd")
         _lib.count_launch()
         return dgu.view(ctx.shape)

@@ -106,18 +106,9 @@ def gemm(
             return out
     if bn == 0:
         bn = _tile_plan(M, N)
-    lib = _lib.kernels()
-    fn = lib.b200_gemm_bf16
-    fn.restype = ctypes.c_int
-    rc = fn(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias),
-        ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-        ctypes.c_longlong(a.stride(0)), ctypes.c_longlong(b.stride(0)),
-        ctypes.c_longlong(out.stride(0)),
-        ctypes.c_int(int(a_mn)), ctypes.c_int(int(b_mn)),
-        ctypes.c_int(int(out.dtype == torch.float32)), ctypes.c_int(int(accumulate)),
-        ctypes.c_int(bn), _lib.stream_ptr(),
-    )
+    rc = _lib.bind("b200_gemm_bf16", "pppp iii lll iiiii p")(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.addr(bias), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+        a_mn, b_mn, out.dtype == torch.float32, accumulate, bn, _lib.stream_raw())
     _lib.check(rc, "b200_gemm_bf16")
     _lib.count_launch()
     return out
