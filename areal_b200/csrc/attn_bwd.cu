@@ -24,7 +24,9 @@
 // their hand-offs take four times as long, so the roles overlap: S^T of the next block is issued as soon as P^T is
 // consumed and is ready while the compute warps still work on dS^T; four warps of their own drain dQ while
 // dK accumulates. Before, one warp set did everything in turn: 8 sequences of 8192, 16 / 8 heads: 11.6 ms (472
-// TFLOP/s), now 6.7 ms (825 TFLOP/s).
+// TFLOP/s), now 6.5 ms (842 TFLOP/s). The tensor cores
+// are busy 42% of the time: what is left is the chain from dS^T over dQ and its read-out to the next dP^T (taking dQ out by bulk
+// copies from shared memory, or not at all, changes nothing).
 //
 // Replaces flash-attn's backward / aten._flash_attention_backward in the
 // reference (areal/experimental/models/archon/attention/varlen.py:116).
@@ -109,6 +111,36 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       : "memory");
 }
 
+// One arrival for the warp: 32 lanes that arrive by themselves queue up at the barrier.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)),
+        "l"(reinterpret_cast<const uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return d;
+}
+
 // What a compute thread needs to know to mask its key row against a query block.
 struct BwdMask {
   bool kv_valid, diag;
@@ -128,12 +160,13 @@ __device__ __forceinline__ void bwd_p32(const uint32_t (&raw)[32], const float* 
 #pragma unroll
   for (int e = 0; e < 32; e += 4) {
     const float4 l = *reinterpret_cast<const float4*>(lse + e);
-    const float lv[4] = {l.x, l.y, l.z, l.w};
-    float p[4];
+    const float2 sc = make_float2(scale_log2, scale_log2);
+    const float2 a0 = fma2(make_float2(__uint_as_float(raw[e]), __uint_as_float(raw[e + 1])), sc, make_float2(l.x, l.y));
+    const float2 a1 = fma2(make_float2(__uint_as_float(raw[e + 2]), __uint_as_float(raw[e + 3])), sc, make_float2(l.z, l.w));
+    float p[4] = {exp2_ftz(a0.x), exp2_ftz(a0.y), exp2_ftz(a1.x), exp2_ftz(a1.y)};
+    if (MASK) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      p[u] = exp2_ftz(__uint_as_float(raw[e + u]) * scale_log2 - lv[u]);
-      if (MASK) p[u] = m.valid<TREE>(col0 + e + u) ? p[u] : 0.f;
+      for (int u = 0; u < 4; ++u) p[u] = m.valid<TREE>(col0 + e + u) ? p[u] : 0.f;
     }
     __nv_bfloat162 a = __floats2bfloat162_rn(p[0], p[1]), b = __floats2bfloat162_rn(p[2], p[3]);
     packed[e / 2] = *reinterpret_cast<uint32_t*>(&a);
@@ -201,15 +234,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&q_empty[i], 1);
       mbar_init(&do_full[i], 1);
       mbar_init(&do_empty[i], 1);
-      mbar_init(&ls_full[i], kBwdDrain * 32);
+      mbar_init(&ls_full[i], kBwdDrain);
     }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_ready, kBwdCompute * 32);
-    mbar_init(ds_ready, kBwdCompute * 32);
+    mbar_init(p_ready, kBwdCompute);
+    mbar_init(ds_ready, kBwdCompute);
     mbar_init(ds_free, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_read, kBwdDrain * 32);
+    mbar_init(dq_read, kBwdDrain);
     mbar_init(acc_done, 1);
     fence_mbar_init();
     prefetch_tmap(&tmQ);
@@ -276,13 +309,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t id_kmn = make_idesc(1, 1, 0, 1, kBT, kD);  // A K-major, B MN-major
       constexpr uint32_t id_mnmn = make_idesc(1, 1, 1, 1, kD, kBT); // both MN-major
       constexpr uint32_t HALF = kTileBytes / 2;
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sdS);
+      // Descriptors of the tiles, once; a reduction step, the second half and the other stage are additions to the address
+      // field. One thread issues 40 products a block, and building two descriptors for each held it up.
+      constexpr uint32_t kStage = kTileBytes >> 4;
+      auto k_major = [](const uint8_t* t) { return make_sdesc_sw128(smem_u32(t), 16, 1024); };
+      auto mn_major = [](const uint8_t* t) { return make_sdesc_sw128(smem_u32(t), HALF, 1024); };
+      const uint64_t dK_k = k_major(sK), dK_mn = mn_major(sK), dV_k = k_major(sV), dS_k = k_major(sdS), dS_mn = mn_major(sdS);
+      const uint64_t dQ_k = k_major(sQ), dQ_mn = mn_major(sQ), dO_k = k_major(sdO), dO_mn = mn_major(sdO);
       // D[128 keys, 128 queries] = tile (K-major) * rows of stage (K-major)^T
-      auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
+      auto scores = [&](uint32_t d, uint64_t a, uint64_t b) {
 #pragma unroll
         for (int k = 0; k < kD / 16; ++k) {
-          const uint32_t off = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(d, make_sdesc_sw128(a + off, 16, 1024), make_sdesc_sw128(b + off, 16, 1024), id_kk, k > 0 ? 1u : 0u);
+          const uint32_t off = ((k >> 2) * HALF + (k & 3) * 32) >> 4;
+          umma_f16(d, a + off, b + off, id_kk, k > 0 ? 1u : 0u);
         }
       };
       bool ok = mbar_wait(kv_full, 0, abort_flag);
@@ -290,13 +329,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ok = mbar_wait(&q_full[0], 0, abort_flag);
         tc_fence_after();
         if (ok) {
-          scores(tm_S, k_addr, smem_u32(sQ));
+          scores(tm_S, dK_k, dQ_k);
           umma_commit(s_full);
           ok = mbar_wait(&do_full[0], 0, abort_flag);
           tc_fence_after();
         }
         if (ok) {
-          scores(tm_dP, v_addr, smem_u32(sdO));
+          scores(tm_dP, dV_k, dO_k);
           umma_commit(dp_full);
         }
       }
@@ -305,34 +344,30 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t nph = ((it + 1) >> 1) & 1;
         const uint32_t itp = it & 1;
         const bool more = it + 1 < n_iter;
-        const uint32_t q_addr = smem_u32(sQ + st * kTileBytes);
-        const uint32_t do_addr = smem_u32(sdO + st * kTileBytes);
         if (!mbar_wait(p_ready, itp, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < kBT / 16; ++k)  // dV += P^T dO   (reduction over q rows)
-          umma_f16_ts(tm_dV, tm_S + (k >> 2) * 64 + (k & 3) * 8, make_sdesc_sw128(do_addr + k * 2048, HALF, 1024), id_kmn,
+          umma_f16_ts(tm_dV, tm_S + (k >> 2) * 64 + (k & 3) * 8, dO_mn + st * kStage + k * 128, id_kmn,
                       (it > 0 || k > 0) ? 1u : 0u);
         umma_commit(&do_empty[st]);
         if (more) {
           // products run in the order of issue: S^T of the next block overwrites P^T when dV has read it
           if (!mbar_wait(&q_full[nst], nph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          scores(tm_S, k_addr, smem_u32(sQ + nst * kTileBytes));
+          scores(tm_S, dK_k, dQ_k + nst * kStage);
           umma_commit(s_full);
         }
         if (!mbar_wait(ds_ready, itp, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < kBT / 16; ++k)  // dQ^T = K^T dS^T  (reduction over kv rows)
-          umma_f16(tm_dP, make_sdesc_sw128(k_addr + k * 2048, HALF, 1024), make_sdesc_sw128(ds_addr + k * 2048, HALF, 1024),
-                   id_mnmn, k > 0 ? 1u : 0u);
+          umma_f16(tm_dP, dK_mn + k * 128, dS_mn + k * 128, id_mnmn, k > 0 ? 1u : 0u);
         umma_commit(dq_full);
 #pragma unroll
         for (int k = 0; k < kBT / 16; ++k) {  // dK += dS^T Q
-          const uint32_t aoff = (k >> 2) * HALF + (k & 3) * 32;
-          umma_f16(tm_dK, make_sdesc_sw128(ds_addr + aoff, 16, 1024), make_sdesc_sw128(q_addr + k * 2048, HALF, 1024), id_kmn,
-                   (it > 0 || k > 0) ? 1u : 0u);
+          const uint32_t aoff = ((k >> 2) * HALF + (k & 3) * 32) >> 4;
+          umma_f16(tm_dK, dS_k + aoff, dQ_mn + st * kStage + k * 128, id_kmn, (it > 0 || k > 0) ? 1u : 0u);
         }
         umma_commit(&q_empty[st]);
         umma_commit(ds_free);
@@ -341,7 +376,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           // the dP^T columns hold dQ^T until it has been read out
           if (!mbar_wait(dq_read, itp, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          scores(tm_dP, v_addr, smem_u32(sdO + nst * kTileBytes));
+          scores(tm_dP, dV_k, dO_k + nst * kStage);
           umma_commit(dp_full);
         }
       }
@@ -361,9 +396,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int qi = i * kBT + d;
       const long long idx = static_cast<long long>(h) * T + tile.seq_start + qi;
       const bool v = qi < tile.seq_len;
-      s_lse[it & 1][d] = v ? lse[idx] * 1.4426950408889634f : INFINITY;
-      s_delta[it & 1][d] = v ? delta[idx] : 0.f;
-      mbar_arrive(&ls_full[it & 1]);
+      s_lse[it & 1][d] = v ? lse[idx] * -1.4426950408889634f : -INFINITY;
+      s_delta[it & 1][d] = v ? -delta[idx] : 0.f;
+      warp_arrive(&ls_full[it & 1]);
     };
     bool ok = true;
     if (n_iter > 0) stage(0);
@@ -386,7 +421,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_wait();
         if (c) {
           tc_fence_before();
-          mbar_arrive(dq_read);
+          warp_arrive(dq_read);
         }
         if (q_rows == kBT) {
 #pragma unroll
@@ -440,7 +475,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tmem_st_32x32(my_S, p);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(p_ready);
+      warp_arrive(p_ready);
       if (!mbar_wait(dp_full, itp, abort_flag)) { ok = false; break; }
       tc_fence_after();
       // the buffer holds dS^T of the previous block until dQ and dK have read it
@@ -461,8 +496,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int u = 0; u < 4; ++u) {
             const uint32_t w = p[cl * 16 + e / 2 + u];
             const float pa = __uint_as_float(w << 16), pb = __uint_as_float(w & 0xffff0000u);
-            __nv_bfloat162 b = __floats2bfloat162_rn(pa * (__uint_as_float(raw[e + 2 * u]) - dd[2 * u]),
-                                                     pb * (__uint_as_float(raw[e + 2 * u + 1]) - dd[2 * u + 1]));
+            const float2 pp = make_float2(pa, pb);
+            const float2 ds = mul2(pp, add2(make_float2(__uint_as_float(raw[e + 2 * u]), __uint_as_float(raw[e + 2 * u + 1])),
+                                            make_float2(dd[2 * u], dd[2 * u + 1])));
+            __nv_bfloat162 b = __floats2bfloat162_rn(ds.x, ds.y);
             o[u] = *reinterpret_cast<uint32_t*>(&b);
           }
           const int piece = cl * 4 + e / 8;
@@ -471,7 +508,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(ds_ready);
+      warp_arrive(ds_ready);
     }
     // epilogue: dK, dV
     if (ok) ok = mbar_wait(acc_done, 0, abort_flag);
