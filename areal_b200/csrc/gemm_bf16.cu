@@ -378,10 +378,9 @@ struct GroupedWgradEpi {
   }
 };
 
-template <bool B_MN>
-static int launch_grouped(const void* A, const void* B, void* C, const int* tile_expert, const int* num_vm,
-                          int max_rows, int E, int N, int K, const int* src_of, cudaStream_t stream) {
-  constexpr int BN = 128;
+template <bool B_MN, int BN>
+static int launch_grouped_bn(const void* A, const void* B, void* C, const int* tile_expert, const int* num_vm,
+                             int max_rows, int E, int N, int K, const int* src_of, cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   CUtensorMap tmA, tmB;
   int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, max_rows, K, (long long)K * 2, kBM, 64);
@@ -408,6 +407,20 @@ static int launch_grouped(const void* A, const void* B, void* C, const int* tile
   return 0;
 }
 
+
+// 256 columns a tile halve what is read of A; with fewer than eight rounds of such tiles (counted with the padding that experts may need) the last one costs more.
+// 96000 rows of 128 experts: 2048 -> 1536 columns 584 -> 528 us, 768 -> 2048 379 -> 322 us, their input gradients 626 -> 548 and 341 ->
+// 276 us, weight gradients 1016 -> 908 and 510 -> 442 us; 5600 rows: 147 us by either.
+static bool grouped_wide(long long rows, int N) {
+  return N >= 256 && rows / kBM * (N / 256) >= 8ll * sm_count();
+}
+
+template <bool B_MN>
+static int launch_grouped(const void* A, const void* B, void* C, const int* tile_expert, const int* num_vm,
+                          int max_rows, int E, int N, int K, const int* src_of, cudaStream_t stream) {
+  auto go = grouped_wide(max_rows, N) ? launch_grouped_bn<B_MN, 256> : launch_grouped_bn<B_MN, 128>;
+  return go(A, B, C, tile_expert, num_vm, max_rows, E, N, K, src_of, stream);
+}
 
 // ------------------------------------------------------------------------------ split-K --
 // Skinny products (a decode step: M <= a few hundred rows against a large weight) are a read of the weight. Its rows are
@@ -825,14 +838,12 @@ int b200_gemm_grouped_glu(const void* A, const void* B, void* C, const int* tile
   return 0;
 }
 
-// Grouped wgrad: dW[e] (+)= dY_e^T X_e with dY [max_rows, N], X [max_rows, K] in the padded layout
-// (padding rows zero) and dW stacked [E, N, K] (fp32 when out_fp32). N % 128 == 0, K % 8 == 0.
-int b200_gemm_grouped_wgrad(const void* dY, const void* X, void* dW, const int* prow0, int max_rows, int E, int N,
+}  // extern "C"
+
+template <int BN>
+static int launch_grouped_wgrad(const void* dY, const void* X, void* dW, const int* prow0, int max_rows, int E, int N,
                             int K, int out_fp32, int accumulate, cudaStream_t stream) {
   using namespace b200;
-  if (E <= 0 || N <= 0 || K <= 0) return 0;
-  if ((N % 128) || (K & 7)) return -100;
-  constexpr int BN = 128;
   using Cfg = GemmCfg<BN>;
   CUtensorMap tmA, tmB;
   int rc = make_tmap_2d(&tmA, dY, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, max_rows, N, (long long)N * 2, 64, 64);
@@ -873,6 +884,18 @@ int b200_gemm_grouped_wgrad(const void* dY, const void* X, void* dW, const int* 
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(tmA, tmB, M, K, max_rows, epi, status);
   B200_CHECK(cudaGetLastError());
   return 0;
+}
+
+extern "C" {
+
+// Grouped wgrad: dW[e] (+)= dY_e^T X_e with dY [max_rows, N], X [max_rows, K] in the padded layout
+// (padding rows zero) and dW stacked [E, N, K] (fp32 when out_fp32). N % 128 == 0, K % 8 == 0.
+int b200_gemm_grouped_wgrad(const void* dY, const void* X, void* dW, const int* prow0, int max_rows, int E, int N,
+                            int K, int out_fp32, int accumulate, cudaStream_t stream) {
+  if (E <= 0 || N <= 0 || K <= 0) return 0;
+  if ((N % 128) || (K & 7)) return -100;
+  auto go = b200::grouped_wide(static_cast<long long>(E) * N, K) ? launch_grouped_wgrad<256> : launch_grouped_wgrad<128>;
+  return go(dY, X, dW, prow0, max_rows, E, N, K, out_fp32, accumulate, stream);
 }
 
 }  // extern "C"
