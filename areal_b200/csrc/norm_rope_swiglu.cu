@@ -122,9 +122,9 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres); one partial row of dw per block. A thread keeps its columns over all
 // rows of its group, so dw accumulates in registers; the next row is loaded before the current one is reduced, so that
 // the barrier of the sum does not leave memory idle. 16384 x 2048: 164 us with a warp a row (8 vectors a lane and no
-// load ahead), 80 us so; 32768 x 4096: 1050 us and 297 us.
+// load ahead), 74 us so (80 when the converted numbers stay in registers across the sum); 32768 x 4096: 1050 us and 283 us.
 template <int VPT>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
@@ -134,11 +134,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   const int tid = threadIdx.x, group = blockDim.x, slot = threadIdx.y;
   const int nvec = H >> 3;
   const float inv_h = 1.f / H;
-  float wv[VPT][8], dwacc[VPT][8];
+  float dwacc[VPT][8];
+  BF8 wv[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = tid + group * i;
-    if (c < nvec) bf8_to_float(reinterpret_cast<const BF8*>(w)[c], wv[i]);
+    if (c < nvec) wv[i] = reinterpret_cast<const BF8*>(w)[c];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
   }
@@ -147,6 +148,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     float rs;
   };
   auto load = [&](long long row, Row& o) {
+    if (row >= T) return;
     o.rs = rstd[row];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -160,22 +162,24 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   };
   const long long step = static_cast<long long>(gridDim.x) * blockDim.y;
   long long row = static_cast<long long>(blockIdx.x) * blockDim.y + slot;
-  Row cur, nxt;
-  if (row < T) load(row, cur);
+  Row next;
+  load(row, next);
   for (int it = 0; row < T; row += step, ++it) {
-    if (row + step < T) load(row + step, nxt);
-    float g[VPT][8], xh[VPT][8], dot = 0.f;
+    const Row cur = next;
+    load(row + step, next);
+    float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       if (tid + group * i < nvec) {
-        bf8_to_float(cur.g[i], g[i]);
-        bf8_to_float(cur.x[i], xh[i]);
+        float g[8], xh[8], f[8];
+        bf8_to_float(cur.g[i], g);
+        bf8_to_float(cur.x[i], xh);
+        bf8_to_float(wv[i], f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] *= cur.rs;
-          dwacc[i][j] += g[i][j] * xh[i][j];
-          g[i][j] *= wv[i][j];
-          dot += g[i][j] * xh[i][j];
+          xh[j] *= cur.rs;
+          dwacc[i][j] += g[j] * xh[j];
+          dot += g[j] * f[j] * xh[j];
         }
       }
     }
@@ -184,9 +188,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     for (int i = 0; i < VPT; ++i) {
       const int c = tid + group * i;
       if (c < nvec) {
-        float o[8];
+        float g[8], xh[8], f[8], o[8];
+        bf8_to_float(cur.g[i], g);
+        bf8_to_float(cur.x[i], xh);
+        bf8_to_float(wv[i], f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = cur.rs * (g[i][j] - xh[i][j] * dot);
+        for (int j = 0; j < 8; ++j) o[j] = cur.rs * (g[j] * f[j] - xh[j] * cur.rs * dot);
         if (dres) {
           float r[8];
           bf8_to_float(cur.r[i], r);
@@ -196,7 +203,6 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         reinterpret_cast<BF8*>(dx + row * H)[c] = float_to_bf8(o);
       }
     }
-    cur = nxt;
   }
   // the block's row groups meet in shared memory
   if (blockDim.y > 1) {
@@ -251,7 +257,7 @@ colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ ou
 // columns 8l..8l+7 and their partners 64 + 8l.. (16-byte vectors), so a warp works on four heads of a token at a time,
 // the sum of squares takes three shuffles, and the token's angles are read once for all of them. With a warp a head and four columns
 // a lane the kernels were bound by issue slots: 16384 tokens of 16 + 8 heads took 91 us forward and 172 us backward, now
-// 51 and 143 us (the latter with the copy of dv, which was a launch of its own).
+// 51 and 119 us (the latter with the copy of dv, which was a launch of its own, and with the next token loaded ahead: 144 without).
 constexpr int kRopeD = 128;
 constexpr int kRopeHeads = 4;  // heads of a warp at a time
 
@@ -425,19 +431,41 @@ qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16
   for (int j = 0; j < 8; ++j) acc.a[j] = acc.b[j] = 0.f;
   RopeVec ww;
   if (has_norm) ww.read(is_q ? qw : kw, l);
-  if (gw < walkers * groups)
+  struct Token {
+    BF8 ga, gb, xa, xb;
+    float rs;
+    int pos;
+  };
+  auto load = [&](int t, Token& o) {
+    if (t >= T) return;
+    const __nv_bfloat16* g = g0 + t * gpitch;
+    o.ga = reinterpret_cast<const BF8*>(g)[l];
+    o.gb = reinterpret_cast<const BF8*>(g + 64)[l];
+    o.pos = pos[t];
+    o.rs = 0.f;
+    if (has_norm) {
+      const __nv_bfloat16* xp = qkv + (static_cast<long long>(t) * all + hs) * D;
+      o.xa = reinterpret_cast<const BF8*>(xp)[l];
+      o.xb = reinterpret_cast<const BF8*>(xp + 64)[l];
+      if (!is_v) o.rs = rstd[static_cast<long long>(t) * heads + h];
+    }
+  };
+  Token next;
+  if (gw < walkers * groups) {
+    load(gw / groups, next);
     for (int t = gw / groups; t < T; t += walkers) {
-      const __nv_bfloat16* g = g0 + t * gpitch;
-      const BF8 raw_a = reinterpret_cast<const BF8*>(g)[l], raw_b = reinterpret_cast<const BF8*>(g + 64)[l];
-      const long long row = static_cast<long long>(t) * all;
-      RopeVec x;
-      float rs = 0.f;
-      if (has_norm) {
-        x.read(qkv + (row + hs) * D, l);
-        rs = is_v ? 0.f : rstd[static_cast<long long>(t) * heads + h];
-      }
+      const Token cur = next;
       RopeAngles r;
-      r.read(cos_t, sin_t, pos[t], l);
+      r.read(cos_t, sin_t, cur.pos, l);
+      load(t + walkers, next);  // on its way while this token is worked on
+      const BF8 raw_a = cur.ga, raw_b = cur.gb;
+      const long long row = static_cast<long long>(t) * all;
+      const float rs = cur.rs;
+      RopeVec x;
+      if (has_norm) {
+        bf8_to_float(cur.xa, x.a);
+        bf8_to_float(cur.xb, x.b);
+      }
       RopeVec d;
       {
         float ga[8], gb[8];
@@ -477,6 +505,7 @@ qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16
         d.write(out, l);
       }
     }
+  }
   if (!has_norm) return;
   if (!is_v) {
     float* sw = s_dw[is_q ? 0 : 1];
