@@ -275,6 +275,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::kTmemCols));
   }
+  // A pair's allocation is given back in both SMs: a CTA that left first would let a kernel of another stream allocate on its
+  // SM while the other CTA is still at it.
+  __syncwarp();
+  cluster_sync_all();
 }
 
 // Host side: tensor maps with boxes of 128 rows (K-major) or 64 x 64 (MN-major) of both operands.
